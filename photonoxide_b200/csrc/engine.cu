@@ -95,7 +95,8 @@ struct StepArgs {
   const T *psi_h_in;
   T *psi_h_out;
   T *psi_e;
-  // sources: per (tile, k) the groups on H (over the H region) and on E (over the tile)
+  // sources: per (tile, k) the groups on H (over the H region) and on E (over the tile); for the
+  // quad kernel per (tile, k, row of the tile's WARPS)
   const int *hbucket;
   const int *ebucket;
   const Group *hgroups;
@@ -1426,6 +1427,53 @@ __device__ __forceinline__ void xcoop(const StepArgs<T> &A, int k, int my, int x
   }
 }
 
+// The sources of one field at a warp's row and plane: its groups g0 .. g1-1, a lane a group (each
+// group a value of its own, its entries in CPU order). The lanes' values go through `rows`, the
+// warp's three scratch rows (component c at rows + c * stride), where the lane that takes a group
+// finds its value wherever it is; with no groups (nearly every row) nothing happens. What bounds
+// it is the chain of loads group -> entry -> waveform, so the groups of a row run side by side:
+// taken one after another by every thread of the CTA, a plane wave's box around 320 x 260 cells
+// took 654 us a step and the 46 080 couplings of a 48 x 48 x 120 Bloch cell 597 us a part.
+template <typename T, int FIELD>
+__device__ __forceinline__ void inject_row(const StepArgs<T> &A, int g0, int g1, T *rows, int stride,
+                                           const T *cb, int cb_stride, int lane, T v[3][4]) {
+  if (g1 <= g0) return;
+  using quad::ROW;
+  using quad::VEC;
+  const Group *groups = FIELD == 1 ? A.hgroups : A.egroups;
+  __syncwarp();  // the lanes are done with the scratch rows' earlier values
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    Vec4<T> o;
+#pragma unroll
+    for (int j = 0; j < 4; j++) o.v[j] = v[c][j];
+    st4(rows + c * stride + VEC * lane, o);
+  }
+  __syncwarp();
+  for (int g = g0 + lane; g < g1; g += 32) {
+    const Group gr = groups[g];
+    const int pos = gr.local % ROW;
+    T *at = rows + gr.comp * stride + pos;
+    T x = *at;
+    if (FIELD == 1) {
+      for (int q = gr.first; q < gr.first + gr.count; q++)
+        x = apply_h<T>(x, A.entries[q], A.waves_h, A.dt);
+    } else {
+      const T cbv = cb[gr.comp * cb_stride + pos];
+      for (int q = gr.first; q < gr.first + gr.count; q++)
+        x = apply_e<T>(x, A.entries[q], A.waves_e, cbv);
+    }
+    *at = x;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const Vec4<T> o = ld4(rows + c * stride + VEC * lane);
+#pragma unroll
+    for (int j = 0; j < 4; j++) v[c][j] = o.v[j];
+  }
+}
+
 // Member q's ADE update (src/fdtd/media.rs:661-705), after the step has written E^{n+1} (curl,
 // slabs and currents) into e_out: J_p^{n+1} = alpha J_p^n + xi J_p^{n-1} + gamma (E^{n+1} -
 // E^{n-1}) / (2 dt) with E^{n+1} corrected by the currents' chi; E^n from e_in kept as E^{n-1}.
@@ -1543,8 +1591,9 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
   }
   const int rowoff = my >= 0 ? my * nx : 0;  // in-plane offsets fit an int (quad_ok)
   // whether the tile has currents in any plane (most have none: then no plane looks them up)
-  const bool hcur = A.hbucket[(long long)tile * nz] != A.hbucket[(long long)tile * nz + nz];
-  const bool ecur = A.ebucket[(long long)tile * nz] != A.ebucket[(long long)tile * nz + nz];
+  const long long tile_rows = (long long)tile * nz * WARPS;
+  const bool hcur = A.hbucket[tile_rows] != A.hbucket[tile_rows + (long long)nz * WARPS];
+  const bool ecur = A.ebucket[tile_rows] != A.ebucket[tile_rows + (long long)nz * WARPS];
 
   // -- copies: warp w copies E's row w, H's row w and cb's row w-1 of a plane, lane l the chunks
   // of its four places; warp 0 (the halo row, which has no E to update) also E's row RW+1 and
@@ -1682,26 +1731,11 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
     }
     // beyond a wall H comes out zero (E's back differences read zero there): its E and H were
     // staged as zeros and its kappa/h is zero, so every term above is +0
-    // the magnetic currents at this tile and plane, each value's entries in CPU order
-    const int bucket = tile * nz + k;
-    const int g0 = hcur ? A.hbucket[bucket] : 0, g1 = hcur ? A.hbucket[bucket + 1] : 0;
-    for (int g = g0; g < g1; g++) {
-      Group gr = A.hgroups[g];
-      const int gw = gr.local / ROW, gi = gr.local % ROW;
-      if (gw == w && (gi >> 2) == lane) {
-        const int jj = gi & 3;
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-#pragma unroll
-          for (int j = 0; j < 4; j++)
-            if (gr.comp == c && jj == j) {
-              T v = hn[c][j];
-              for (int q = gr.first; q < gr.first + gr.count; q++) {
-                v = apply_h<T>(v, A.entries[q], A.waves_h, A.dt);
-              }
-              hn[c][j] = v;
-            }
-      }
+    // the magnetic currents of the row: scratch, the warp's rows of the old H (in registers, ho)
+    if (hcur) {
+      const long long bucket = ((long long)tile * nz + k) * WARPS + w;
+      inject_row<T, 1>(A, A.hbucket[bucket], A.hbucket[bucket + 1], const_cast<T *>(Hrow(sh, 0)),
+                       WARPS * ROW, nullptr, 0, lane, hn);
     }
   };
 
@@ -1905,27 +1939,12 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
                              {cb[2].v[0], cb[2].v[1], cb[2].v[2], cb[2].v[3]}};
         cpml4<T, 0>(A, k, my, mxb, sxl, xmixed, inx, zs, sy, true, en, diff, cbs, sXC + VEC * lane);
       }
-      // the electric currents (src/fdtd.rs:1375-1387)
-      const int bucket = tile * nz + k;
-      const int g0 = ecur ? A.ebucket[bucket] : 0, g1 = ecur ? A.ebucket[bucket + 1] : 0;
-      for (int g = g0; g < g1; g++) {
-        Group gr = A.egroups[g];
-        const int gw = gr.local / ROW, gi = gr.local % ROW;
-        if (gw == w && (gi >> 2) == lane) {
-          const int jj = gi & 3;
-#pragma unroll
-          for (int c = 0; c < 3; c++)
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-              if (gr.comp == c && jj == j) {
-                T v = en[c][j];
-                const T cbv = cb[c].v[j];
-                for (int q = gr.first; q < gr.first + gr.count; q++) {
-                  v = apply_e<T>(v, A.entries[q], A.waves_e, cbv);
-                }
-                en[c][j] = v;
-              }
-        }
+      // the electric currents of the row (src/fdtd.rs:1375-1387)
+      if (ecur) {
+        const long long bucket = ((long long)tile * nz + k) * WARPS + w;
+        inject_row<T, 0>(A, A.ebucket[bucket], A.ebucket[bucket + 1],
+                         const_cast<T *>(Hrow(hb_cur, 0)), WARPS * ROW, Brow(hb_cur, 0), RW * ROW,
+                         lane, en);
       }
       if (lane >= 1 && rowh && mxb >= 0 && xb < nx) {
 #pragma unroll
@@ -2713,9 +2732,12 @@ std::vector<int> quad_order(const fdtd_ctx *c) {
   return order;
 }
 
+// The rows of a tile that the source tables tell apart: the quad kernel's, a warp each.
+int bucket_rows(const fdtd_ctx *c) { return c->quad ? quad::WARPS : 1; }
+
 // Empty source tables: every bucket empty.
 int empty_sources(fdtd_ctx *c) {
-  long long nb = (long long)c->tiles_x * c->tiles_y * c->n[2] + 1;
+  long long nb = (long long)c->tiles_x * c->tiles_y * c->n[2] * bucket_rows(c) + 1;
   std::vector<int> zero(nb, 0);
   release(c, c->hbucket);
   release(c, c->ebucket);
@@ -3332,6 +3354,7 @@ int fdtd_set_sources(fdtd_ctx *c, int32_t nwaves, const fdtd_waveform *waves, in
   // Group by value in CPU order (Resident::plan, resident.rs:546-590), then by (tile, plane):
   // an H value also goes to the tiles whose low halo row or column it is.
   struct Item { long long key; int local; int comp; std::vector<int> entries; };
+  const int brows = bucket_rows(c);
   std::vector<Entry> entries;
   std::vector<std::vector<Item>> per_field(2);
   for (int f = 0; f < 2; f++) {
@@ -3371,7 +3394,7 @@ int fdtd_set_sources(fdtd_ctx *c, int32_t nwaves, const fdtd_waveform *waves, in
       int tx = i / tw, ty = j / th;
       auto push = [&](int ttx, int tty, int lx, int ly, int width) {
         Item it;
-        it.key = ((long long)(tty * c->tiles_x + ttx)) * nz + k;
+        it.key = (((long long)(tty * c->tiles_x + ttx)) * nz + k) * brows + (brows > 1 ? ly : 0);
         it.local = ly * width + lx;
         it.comp = comp;
         it.entries = lists[g];
@@ -3395,7 +3418,7 @@ int fdtd_set_sources(fdtd_ctx *c, int32_t nwaves, const fdtd_waveform *waves, in
       }
     }
   }
-  long long nb = (long long)c->tiles_x * c->tiles_y * nz + 1;
+  long long nb = (long long)c->tiles_x * c->tiles_y * nz * brows + 1;
   std::vector<Entry> ordered_entries;
   std::vector<Group> groups[2];
   std::vector<int> buckets[2];
