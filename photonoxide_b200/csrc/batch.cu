@@ -576,19 +576,11 @@ __global__ void te_contract_kernel(const TeInst<T> *insts, const RecItem *items,
   const TeInst<T> &I = insts[it.inst];
   const long long v = it.index;
   const SeriesDev s = I.series[I.value_series[v]];
-  const long long o = v - s.value0;
-  for (int k = 0; k < s.nf; k++) {
-    double *acc = I.sums + 2 * (s.sum0 + (long long)k * s.volume + o);
-    double re = acc[0], im = acc[1];
-    const double *ph = phase + 2 * ((long long)I.slot0 + s.slot0 + k);
-    for (int m = 0; m < count; m++) {
-      const double x = (double)ring[(long long)m * nring + it.col];
-      re = re + x * ph[2 * (long long)m * nslots_total];
-      im = im + x * ph[2 * (long long)m * nslots_total + 1];
-    }
-    acc[0] = re;
-    acc[1] = im;
-  }
+  const int f0 = blockIdx.y * DFT_F;
+  if (f0 >= s.nf) return;
+  transform_value<T>(ring + it.col, nring, count, phase + 2 * ((long long)I.slot0 + s.slot0 + f0),
+                     nslots_total, I.sums + 2 * (s.sum0 + (long long)f0 * s.volume + (v - s.value0)),
+                     s.volume, s.nf - f0);
 }
 
 // After `count` steps: each instance's step index, copy and record row move on.
@@ -903,6 +895,7 @@ struct fdtd_batch {
   int *d_point = nullptr;
   int2 *d_wave_items = nullptr, *d_slot_items = nullptr;
   int nwave_items = 0, nslot_items = 0, nwaves_total = 0, nslots_total = 0;
+  int freq_chunks = 1;  // the most frequencies of a transform, in chunks of DFT_F
   double *d_waves_h = nullptr, *d_waves_e = nullptr, *d_phase = nullptr;
   RecItem *d_rec = nullptr;
   long long nrec = 0;
@@ -1159,6 +1152,8 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
     for (int p = 0; p < v.nprobes; p++) rec.push_back(RecItem{(int)i, 1, p, -1});
   }
   b->ntiles = (int)tile_inst.size();
+  b->freq_chunks = 1;
+  for (const InstanceView &v : views) b->freq_chunks = std::max(b->freq_chunks, v.freq_chunks);
   b->nwaves_total = (int)waves.size();
   b->nslots_total = slots;
   b->nwave_items = (int)wave_items.size();
@@ -1264,7 +1259,8 @@ void enqueue(fdtd_batch *b, int count) {
     }
   }
   if (b->nring > 0 && b->record) {
-    te_contract_kernel<T><<<(unsigned)((b->nrec + 127) / 128), 128, 0, b->stream>>>(
+    te_contract_kernel<T><<<dim3((unsigned)((b->nrec + 127) / 128), b->freq_chunks), 128, 0,
+                            b->stream>>>(
         insts, b->d_rec, b->nrec, (const T *)b->d_ring, b->nring, b->d_phase, b->nslots_total,
         count);
     b->launches++;

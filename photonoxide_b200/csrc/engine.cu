@@ -2157,27 +2157,21 @@ __global__ void phase_kernel(const double *omega, const int *slot_field, int nsl
 // Sets a captured batch's first step index.
 __global__ void set_base_kernel(long long *base, long long first) { *base = first; }
 
-// sums[f][v] += sum_m ring[m][v] * phase[m][slot(f)], m in time order, f64 (monitors.rs:185-206).
+// sums[f][v] += sum_m ring[m][v] * phase[m][slot(f)], m in time order, f64 (monitors.rs:185-206):
+// a thread a value and DFT_F of its frequencies (blockIdx.y).
 template <typename T>
-__global__ void dft_kernel(const SeriesDev *series, int nseries, const long long *value_series,
-                           long long nvalues, const T *ring, int batch, const double *phase,
-                           int nslots, double *sums) {
-  long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128) dft_kernel(const SeriesDev *series,
+                                                  const long long *value_series, long long nvalues,
+                                                  const T *ring, int batch, const double *phase,
+                                                  int nslots, double *sums) {
+  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nvalues) return;
-  SeriesDev s = series[value_series[v]];
-  long long o = v - s.value0;
-  for (int f = 0; f < s.nf; f++) {
-    double *acc = sums + 2 * (s.sum0 + (long long)f * s.volume + o);
-    double re = acc[0], im = acc[1];
-    const double *ph = phase + 2 * (long long)(s.slot0 + f);
-    for (int m = 0; m < batch; m++) {
-      double x = (double)ring[(long long)m * nvalues + v];
-      re = re + x * ph[2 * (long long)m * nslots];
-      im = im + x * ph[2 * (long long)m * nslots + 1];
-    }
-    acc[0] = re;
-    acc[1] = im;
-  }
+  const SeriesDev s = series[value_series[v]];
+  const int f0 = blockIdx.y * DFT_F;
+  if (f0 >= s.nf) return;
+  transform_value<T>(ring + v, nvalues, batch, phase + 2 * (long long)(s.slot0 + f0), nslots,
+                     sums + 2 * (s.sum0 + (long long)f0 * s.volume + (v - s.value0)), s.volume,
+                     s.nf - f0);
 }
 
 // The transform of a complex run's values (src/fdtd/monitors.rs:127-154): each step's
@@ -2321,6 +2315,7 @@ struct fdtd_ctx {
   long long *d_where = nullptr, *d_value_series = nullptr;
   SeriesDev *d_series = nullptr;
   int nseries = 0, nslots = 0;
+  int freq_chunks = 1;  // the most frequencies of a series, in chunks of DFT_F
   double *d_omega = nullptr;
   int *d_slot_field = nullptr;
   long long nsums = 0;
@@ -2353,6 +2348,10 @@ struct fdtd_ctx {
   // first such transfer and kept (counted in the HBM budget)
   double *stage = nullptr;
   long long stage_len = 0;
+  // page-locked chunks the transforms' sums are read through, two in turn, made on the first large
+  // read and kept (fdtd_instance_add_dft); sums_fresh: steps have been taken since the last read
+  double *host_stage[2] = {nullptr, nullptr};
+  bool sums_fresh = true;
   // step-kernel timing: pairs of events around each launch while profiling
   bool profiling = false;
   std::vector<cudaEvent_t> events;
@@ -2757,6 +2756,7 @@ int run_impl(fdtd_ctx *c, long long steps, long long first) {
     return fail(c, FDTD_E_STATE, "set the sources again after the plane waves");
   if (c->nbloch > 0)
     return fail(c, FDTD_E_STATE, "a context with Bloch couplings steps with fdtd_bloch_run");
+  c->sums_fresh = true;
   const int K = c->ring_k > 0 ? c->ring_k : 64;
   // the probes' record: grow to the run's steps
   if (c->nprobes > 0 && c->recorded + steps > c->record_cap) {
@@ -2820,9 +2820,9 @@ int run_impl(fdtd_ctx *c, long long steps, long long first) {
       phase_kernel<<<(total + 127) / 128, 128, 0, c->stream>>>(c->d_omega, c->d_slot_field,
                                                                 c->nslots, first + at, base,
                                                                 batch, c->dt, c->phase);
-      dft_kernel<T><<<(unsigned)((c->nvalues + 127) / 128), 128, 0, c->stream>>>(
-          c->d_series, c->nseries, c->d_value_series, c->nvalues, (const T *)c->ring, batch,
-          c->phase, c->nslots, c->sums);
+      dft_kernel<T><<<dim3((unsigned)((c->nvalues + 127) / 128), c->freq_chunks), 128, 0,
+                      c->stream>>>(c->d_series, c->d_value_series, c->nvalues, (const T *)c->ring,
+                                   batch, c->phase, c->nslots, c->sums);
       c->launches += 2;
     }
   };
@@ -2908,6 +2908,7 @@ int bloch_impl(fdtd_ctx *a, fdtd_ctx *b, const std::vector<WrapDev> &hw,
   if (a->N != b->N || a->precision != b->precision || a->nbloch != b->nbloch)
     return fail(a, FDTD_E_INVALID, "the two parts of a complex run differ");
   CUDA_TRY(a, cudaStreamSynchronize(b->stream));
+  a->sums_fresh = b->sums_fresh = true;
   const cudaStream_t st = a->stream;
   const int K = a->ring_k > 0 ? a->ring_k : 64;
   if (int r = grow_record(a, steps)) return r;
@@ -3240,6 +3241,8 @@ void fdtd_destroy(fdtd_ctx *c) {
   if (!c) return;
   if (c->stream) cudaStreamSynchronize(c->stream);
   for (cudaEvent_t ev : c->events) cudaEventDestroy(ev);
+  for (double *p : c->host_stage)
+    if (p) cudaFreeHost(p);
   for (int p = 0; p < 2; p++)
     if (c->graph[p]) cudaGraphExecDestroy(c->graph[p]);
   if (c->stream) {
@@ -3676,6 +3679,8 @@ int fdtd_set_dft(fdtd_ctx *c, int32_t nseries, const fdtd_series *series, int32_
   c->nseries = nseries;
   c->nslots = (int)omega.size();
   c->nsums = sums;
+  c->freq_chunks = 1;
+  for (const SeriesDev &x : sd) c->freq_chunks = std::max(c->freq_chunks, (x.nf + DFT_F - 1) / DFT_F);
   if (values == 0) return 0;
   // the ring: K steps of the values, K as large as 64 while it stays within 1 GB
   long long K = 64;
@@ -4022,6 +4027,7 @@ int fdtd_instance_view(fdtd_ctx *c, InstanceView *v) {
   v->slot_field = c->d_slot_field;
   v->sums = c->sums;
   v->nsums = c->nvalues > 0 ? c->nsums : 0;
+  v->freq_chunks = c->freq_chunks;
   v->nprobes = c->nprobes;
   v->probes = c->d_probes;
   v->media = c->media;
@@ -4053,8 +4059,71 @@ int fdtd_instance_reserve(fdtd_ctx *c, long long steps, double **rows) {
 
 void fdtd_instance_advance(fdtd_ctx *c, long long steps) {
   if (!c) return;
+  c->sums_fresh = true;
   if (steps & 1) c->parity = 1 - c->parity;
   if (c->nprobes > 0) c->recorded += steps;
+}
+
+namespace {
+constexpr long long HOST_CHUNK = 1LL << 19;  // doubles: 4 MiB
+
+// n doubles of src added into the parts laid end to end, from place `at` of them on. Large runs
+// over the host's threads: one core adds at a fraction of what the link delivers.
+void add_into_parts(const double *src, long long at, long long n, int nparts, double *const *parts,
+                    const long long *lens) {
+  long long base = 0;
+  for (int p = 0; p < nparts && base < at + n; base += lens[p], p++) {
+    const long long lo = std::max(at, base), hi = std::min(at + n, base + lens[p]);
+    if (hi <= lo) continue;
+    double *to = parts[p] + (lo - base);
+    const double *from = src + (lo - at);
+    const long long m = hi - lo;
+#pragma omp parallel for schedule(static) if (m > (1 << 16))
+    for (long long q = 0; q < m; q++) to[q] += from[q];
+  }
+}
+}  // namespace
+
+// Read in 4 MiB chunks through two page-locked buffers, one filled while the other is added: a
+// whole-plane transform (400 x 200, six components, 21 frequencies: 161 MB) had gone through three
+// pageable arrays made for each read, twice a call.
+int fdtd_instance_add_dft(fdtd_ctx *c, int nparts, double *const *parts, const long long *lens) {
+  if (!c) return FDTD_E_INVALID;
+  const long long n = 2 * c->nsums;
+  long long room = 0;
+  for (int p = 0; p < nparts; p++) room += lens[p];
+  if (room != n) return fail(c, FDTD_E_INVALID, "the transforms hold %lld sums, not %lld", c->nsums, room / 2);
+  if (n == 0 || !c->sums_fresh) return 0;
+  std::vector<double> plain;  // short reads, and where page-locked memory is refused
+  double *buf[2] = {nullptr, nullptr};
+  if (n > HOST_CHUNK / 8) {
+    for (int b = 0; b < 2; b++)
+      if (!c->host_stage[b] &&
+          cudaHostAlloc((void **)&c->host_stage[b], HOST_CHUNK * 8, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        c->host_stage[b] = nullptr;
+      }
+    buf[0] = c->host_stage[0];
+    buf[1] = c->host_stage[1];
+  }
+  if (!buf[0] || !buf[1]) {
+    plain.resize(2 * std::min(n, HOST_CHUNK));
+    buf[0] = plain.data();
+    buf[1] = plain.data() + plain.size() / 2;
+  }
+  auto get = [&](long long at) {
+    const long long m = std::min(HOST_CHUNK, n - at);
+    return cudaMemcpyAsync(buf[(at / HOST_CHUNK) & 1], c->sums + at, m * 8, cudaMemcpyDeviceToHost, c->stream);
+  };
+  CUDA_TRY(c, get(0));
+  for (long long at = 0; at < n; at += HOST_CHUNK) {
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    if (at + HOST_CHUNK < n) CUDA_TRY(c, get(at + HOST_CHUNK));
+    add_into_parts(buf[(at / HOST_CHUNK) & 1], at, std::min(HOST_CHUNK, n - at), nparts, parts, lens);
+  }
+  CUDA_TRY(c, cudaMemsetAsync(c->sums, 0, c->nsums * 16, c->stream));
+  c->sums_fresh = false;
+  return 0;
 }
 
 int fdtd_fast_division(const fdtd_ctx *c, int32_t out[3]) {

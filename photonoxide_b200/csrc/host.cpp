@@ -25,6 +25,7 @@
 #include "photonoxide_sim.h"
 #include "photonoxide_adjoint.h"
 #include "photonoxide_batch.h"
+#include "instance.h"
 #include "portable.h"
 #include "average.cuh"
 #include "cpml.cuh"
@@ -423,13 +424,14 @@ struct pxs_sim {
   // Adds the device's transform sums into the host's.
   int pull_sums() {
     if (!ctx || !configured || series.empty()) return 0;
-    int64_t total = 0;
-    for (auto &s : series) total += (int64_t)s.sums.size() / 2;
-    std::vector<double> add(2 * total, 0.0);
-    if (int r = fdtd_read_dft(ctx, add.data(), total)) return fail(r, "%s", fdtd_last_error(ctx));
-    int64_t at = 0;
-    for (auto &s : series)
-      for (size_t q = 0; q < s.sums.size(); q++) s.sums[q] += add[at++];
+    std::vector<double *> parts;
+    std::vector<long long> lens;
+    for (auto &s : series) {
+      parts.push_back(s.sums.data());
+      lens.push_back((long long)s.sums.size());
+    }
+    if (int r = fdtd_instance_add_dft(ctx, (int)parts.size(), parts.data(), lens.data()))
+      return fail(r, "%s", fdtd_last_error(ctx));
     return 0;
   }
 
@@ -2379,7 +2381,14 @@ int64_t pxs_transforms(pxs_sim *s, double *out) {
       for (size_t q = F.series0; q < F.series0 + 4; q++) order.push_back(q);
   for (size_t q : order) {
     const Series &sr = s->series[q];
-    if (out) std::copy(sr.sums.begin(), sr.sums.end(), out + 2 * at);
+    if (out) {
+      // over the host's threads where long: the caller's fresh array is paged in as it is written
+      const double *from = sr.sums.data();
+      double *to = out + 2 * at;
+      const int64_t n = (int64_t)sr.sums.size();
+#pragma omp parallel for schedule(static) if (n > (1 << 16))
+      for (int64_t v = 0; v < n; v++) to[v] = from[v];
+    }
     at += (int64_t)sr.sums.size() / 2;
   }
   return at;

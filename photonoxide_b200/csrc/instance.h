@@ -33,6 +33,7 @@ struct InstanceView {
   const int *slot_field;
   double *sums;
   long long nsums;  // complex sums
+  int freq_chunks;  // the most frequencies of a series, in chunks of DFT_F (at least 1)
   int nprobes;
   const long long *probes;
   bool media;
@@ -46,4 +47,8 @@ int fdtd_instance_view(fdtd_ctx *c, InstanceView *v);
 int fdtd_instance_reserve(fdtd_ctx *c, long long steps, double **rows);
 // After `steps` steps taken by the batch: the current copies and the record's length.
 void fdtd_instance_advance(fdtd_ctx *c, long long steps);
+// The transforms' sums since the last read added into `parts` (doubles, interleaved, laid end to
+// end in the layout of fdtd_read_dft; lens: each part's), the device's then zero. Does nothing
+// where no step has been taken since the last read.
+int fdtd_instance_add_dft(fdtd_ctx *c, int nparts, double *const *parts, const long long *lens);
 int fdtd_instance_fail(fdtd_ctx *c, int code, const char *what);
