@@ -45,6 +45,7 @@ constexpr int G = 32;  // steps per chunk (even: a chunk leaves the copies' pari
 template <typename T>
 struct TeInst {
   int nx, ny, px, py;  // sizes, periodic flags
+  int pitch;           // values from a row of a y slab's psi to the next
   long long N;
   T dt, sx, sy;        // the step's dt and the grid steps along x and y, as the kernel rounds them
   T inv_sx, inv_sy;    // 1/step rounded, and whether div_by_step's product form is checked
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(THREADS) te_step_kernel(
           const int side = my < ny / 2 ? 0 : 1;
           const SlabEntry &s = I.hy[side];
           if (in_slab(s, my))
-            hz = slab_h(I, s, my, s.psi + (long long)(my - s.from) * nx + mx, pin, pout, own, dyEx,
+            hz = slab_h(I, s, my, s.psi + (long long)(my - s.from) * I.pitch + mx, pin, pout, own, dyEx,
                         1, T(-1), hz);
         }
       }
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(THREADS) te_step_kernel(
           const int side = y < ny / 2 ? 0 : 1;
           const SlabEntry &s = I.ey[side];
           if (in_slab(s, y))
-            nex = slab_e(I, s, y, s.psi + (long long)(y - s.from) * nx + x, I.psi_e, dyHz, 1,
+            nex = slab_e(I, s, y, s.psi + (long long)(y - s.from) * I.pitch + x, I.psi_e, dyHz, 1,
                          T(1), cbx, nex);
         }
         if (!I.px) {
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(THREADS, 4) te_quad_kernel(
 #pragma unroll
           for (int j = 0; j < 4; j++)
             if (ok[j])
-              hz[j] = slab_h(I, s, my, s.psi + (long long)(my - s.from) * nx + mx[j], pin, pout,
+              hz[j] = slab_h(I, s, my, s.psi + (long long)(my - s.from) * I.pitch + mx[j], pin, pout,
                              own, dyEx[j], 1, T(-1), hz[j]);
       }
 #pragma unroll
@@ -448,7 +449,7 @@ __global__ void __launch_bounds__(THREADS, 4) te_quad_kernel(
 #pragma unroll
           for (int j = 0; j < 4; j++)
             if (ok[j])
-              nex[j] = slab_e(I, s, my, s.psi + (long long)(my - s.from) * nx + mx[j], I.psi_e,
+              nex[j] = slab_e(I, s, my, s.psi + (long long)(my - s.from) * I.pitch + mx[j], I.psi_e,
                               dyHz[j], 1, T(1), cbx.v[j], nex[j]);
       }
       if (!I.px) {
@@ -675,7 +676,7 @@ __global__ void __launch_bounds__(THREADS) te_adjoint_kernel(const TeInst<T> *in
   // psi~ of an E slab value in total: what the later steps carried, plus this step's use of it
   // (E_x += cb (+psi') along y; E_y += cb (-psi') along x)
   auto psi_ex_total = [&](int x, int y, long long r, const SlabEntry &s) -> T {
-    return pei[s.psi + (long long)(y - s.from) * nx + x] + I.cb[r] * eb[r];
+    return pei[s.psi + (long long)(y - s.from) * I.pitch + x] + I.cb[r] * eb[r];
   };
   auto psi_ey_total = [&](int x, int y, long long r, const SlabEntry &s) -> T {
     return pei[s.psi + (long long)y * s.pw + (x - s.pf)] - I.cb[N + r] * eb[N + r];
@@ -685,7 +686,7 @@ __global__ void __launch_bounds__(THREADS) te_adjoint_kernel(const TeInst<T> *in
     return phi[s.psi + (long long)y * s.pw + (x - s.pf)] - I.dt * hbar;
   };
   auto psi_hy_total = [&](int x, int y, T hbar, const SlabEntry &s) -> T {
-    return phi[s.psi + (long long)(y - s.from) * nx + x] + I.dt * hbar;
+    return phi[s.psi + (long long)(y - s.from) * I.pitch + x] + I.dt * hbar;
   };
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int x0 = (t % I.tiles_x) * TW, y0 = (t / I.tiles_x) * TH;
@@ -716,7 +717,7 @@ __global__ void __launch_bounds__(THREADS) te_adjoint_kernel(const TeInst<T> *in
           if (in_slab(s0, my)) {
             const T tot = psi_ex_total(mx, my, r, s0);
             acc = acc + coef_a(I, s0, my) / I.sy * tot;
-            if (own) peo[s0.psi + (long long)(my - s0.from) * nx + mx] = coef_b(I, s0, my) * tot;
+            if (own) peo[s0.psi + (long long)(my - s0.from) * I.pitch + mx] = coef_b(I, s0, my) * tot;
           }
           if (myp >= 0) {
             const SlabEntry &s1 = I.ey[myp < ny / 2 ? 0 : 1];
@@ -774,7 +775,7 @@ __global__ void __launch_bounds__(THREADS) te_adjoint_kernel(const TeInst<T> *in
         if (in_slab(s0, y)) {
           const T tot = psi_hy_total(x, y, hc, s0);
           ax = ax - coef_a(I, s0, y) / I.sy * tot;
-          pho[s0.psi + (long long)(y - s0.from) * nx + x] = coef_b(I, s0, y) * tot;
+          pho[s0.psi + (long long)(y - s0.from) * I.pitch + x] = coef_b(I, s0, y) * tot;
         }
         if (ym >= 0) {
           const SlabEntry &s1 = I.hy[ym < ny / 2 ? 0 : 1];
@@ -1011,6 +1012,7 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
     memset(&I, 0, sizeof I);
     I.nx = v.n[0];
     I.ny = v.n[1];
+    I.pitch = v.pitch;
     I.px = v.periodic[0];
     I.py = v.periodic[1];
     I.N = v.N;

@@ -74,6 +74,7 @@ constexpr int quad_max_runs = 64;
 template <typename T>
 struct StepArgs {
   int n[3];
+  int pitch;  // values from one of the psi's rows along x to the next, y and z slabs (n[0] padded)
   long long N;
   int periodic[3];
   int low[3], high[3];
@@ -132,7 +133,7 @@ __device__ inline T slab_update(const StepArgs<T> &A, const SlabEntry *s, int c,
   int m = w == 0 ? i : (w == 1 ? j : k);
   int q = m - s->from;
   int li = i, lj = j, lk = k;
-  int dx = A.n[0], dy = A.n[1];
+  int dx = A.pitch, dy = A.n[1];
   if (w == 0) { li = i - s->pf; dx = s->pw; }
   else if (w == 1) { lj = q; dy = s->count; }
   else lk = q;
@@ -394,6 +395,15 @@ __device__ inline void cp_async_value(T *smem, const T *gmem) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(s), "l"(gmem),
                "n"((int)sizeof(T))
+               : "memory");
+}
+// The same, or a zero where `valid` is false.
+template <typename T>
+__device__ inline void cp_async_value(T *smem, const T *gmem, bool valid) {
+  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  int n = valid ? (int)sizeof(T) : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(s), "l"(gmem),
+               "n"((int)sizeof(T)), "r"(n)
                : "memory");
 }
 // Brings `bytes` (a multiple of 16, from a 16-byte aligned address) of global memory into L2
@@ -745,7 +755,7 @@ __device__ __forceinline__ T slab_apply(const StepArgs<T> &A, const SlabEntry s,
   int m = w == 0 ? i : (w == 1 ? j : k);
   int q = m - s.from;
   int li = i, lj = j, lk = k;
-  int dx = A.n[0], dy = A.n[1];
+  int dx = A.pitch, dy = A.n[1];
   if (w == 0) { li = i - s.pf; dx = s.pw; }
   else if (w == 1) { lj = q; dy = s.count; }
   else lk = q;
@@ -1187,6 +1197,12 @@ struct Smem {
   static constexpr size_t BYTES =
       sizeof(T) * (3 * (size_t)E_SLOT + 2 * (size_t)HB_SLOT + X + XC + FX);
 };
+// CTAs an SM holds: two by shared memory in f32, one in f64 (220 KB), whose threads may then have
+// 255 registers (at the 128 of two CTAs an SM the f64 forms spilled 340 and 428 bytes).
+template <typename T>
+constexpr int ctas() {
+  return sizeof(T) == 4 ? 2 : 1;
+}
 }  // namespace quad
 
 template <typename T>
@@ -1288,8 +1304,8 @@ __device__ __forceinline__ void cpml4(const StepArgs<T> &A, int k, int my, int m
                                       T v[3][4], const T diff[3][3][4], const T cbv[3][4],
                                       const T *xc) {
   // xc: the CTA's x coefficient table at this lane's first place (quad::Smem::XC)
-  const int nx = A.n[0], ny = A.n[1];
-  const long long plane = (long long)nx * ny;
+  const int ny = A.n[1];
+  const long long plane = (long long)A.pitch * ny;
   const T *pin = FIELD == 1 ? A.psi_h_in : A.psi_e;
   T *pout = FIELD == 1 ? A.psi_h_out : A.psi_e;
   const T one = T(1), minus = T(-1);
@@ -1300,14 +1316,14 @@ __device__ __forceinline__ void cpml4(const StepArgs<T> &A, int k, int my, int m
   auto y_slab = [&](int c, T sign, const T d[4], T w[4], const T *cb) {
     const SlabEntry &s = A.slab[FIELD][c][1][sy];
     if (!s.count) return;
-    const long long at = s.psi + ((long long)k * s.count + (my - s.from)) * nx + mxb;
+    const long long at = s.psi + ((long long)k * s.count + (my - s.from)) * A.pitch + mxb;
     slab4_loaded<T, FIELD>(A, pout + at, ld4(pin + at), s, my - s.from, 1, sign, d, w, cb,
                            write);
   };
   auto z_slab = [&](int c, T sign, const T d[4], T w[4], const T *cb) {
     const SlabEntry &s = A.slab[FIELD][c][2][zside];
     if (!s.count) return;
-    const long long at = s.psi + (long long)(k - s.from) * plane + (long long)my * nx + mxb;
+    const long long at = s.psi + (long long)(k - s.from) * plane + (long long)my * A.pitch + mxb;
     slab4_loaded<T, FIELD>(A, pout + at, ld4(pin + at), s, k - s.from, 2, sign, d, w, cb,
                            write);
   };
@@ -1512,8 +1528,13 @@ __global__ void ade_kernel(StepArgs<T> A) {
   if (q < A.media.members) ade_update(A, q);
 }
 
-template <typename T, bool LOSSY>
-__global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
+// RAGGED: nx not a multiple of 4, the grid not periodic along x. A row then starts anywhere, so
+// its values are copied and stored one by one, lane l the places l, l + 32, l + 64 and l + 96 of the
+// row (whole 128-byte lines), and the places after the grid's end are staged as zeros, as those
+// beyond a wall are. Only the copies, the stores and ca's reads differ. Such grids had gone to the
+// row kernel: a pass of 64 steps of a 301 x 157 x 83 block, its sums read, 18.7 ms there and 10.0 here.
+template <typename T, bool LOSSY, bool RAGGED>
+__global__ void __launch_bounds__(quad::THREADS, quad::ctas<T>()) quad_kernel(StepArgs<T> A) {
   using namespace quad;
   using S = Smem<T>;
   constexpr int CH = 16 / (int)sizeof(T);  // values a cp.async chunk carries
@@ -1618,6 +1639,22 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
 #pragma unroll
     for (int q = 0; q < VEC / CH; q++) cp_async16(dst + q * CH, src + q * CH, ok);
   };
+  // a row of ROW places from `row` on (`off`: its first place's offset within a plane, which may
+  // lie before the grid's row; ok: the grid has the row), place by place over the lanes
+  int inrow = 0;  // which of the lane's places l + 32 q the grid's rows have
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int x = x0 - VEC + lane + 32 * q;
+    if (x >= 0 && x < nx) inrow |= 1 << q;
+  }
+  auto whole_row = [&](T *row, const T *field, int off, bool ok, long long pbase) {
+    const T *src = field + pbase + off + lane;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const bool in = ok && pbase >= 0 && (inrow >> q & 1);
+      cp_async_value(row + lane + 32 * q, in ? src + 32 * q : A.e_in, in);
+    }
+  };
   // E(ke) rows into E slot E (ke < 0: zeros); H(kh), cb(kh) rows into HB slot H (H null: none)
   // a lane of the x slab's (xcoop): component y (lanes below P) or z, its place xp0 + xq
   const bool xstage = xco && rowh && lane < 2 * xP;
@@ -1625,22 +1662,40 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
   auto issue = [&](T *E, int ke, T *H, int kh) {
     const long long pe = ke >= 0 ? (long long)ke * plane : -1;
 #pragma unroll
-    for (int c = 0; c < 3; c++) chunk(E + c * ER * EW + erow, A.e_in + c * N, off_e0, pe);
+    for (int c = 0; c < 3; c++) {
+      if (RAGGED)
+        whole_row(E + (c * ER + w) * EW, A.e_in + c * N, rowoff + x0 - VEC, my >= 0, pe);
+      else chunk(E + c * ER * EW + erow, A.e_in + c * N, off_e0, pe);
+    }
     if (w0) {
 #pragma unroll
-      for (int c = 0; c < 3; c++)
-        chunk(E + (c * ER + RW + 1) * EW + VEC * lane, A.e_in + c * N, off_e1, pe);
+      for (int c = 0; c < 3; c++) {
+        T *row = E + (c * ER + RW + 1) * EW;
+        if (RAGGED)
+          whole_row(row, A.e_in + c * N, myp_last * nx + x0 - VEC, myp_last >= 0, pe);
+        else chunk(row + VEC * lane, A.e_in + c * N, off_e1, pe);
+      }
       for (int q = lane; q < 3 * ER; q += 32) {
         const int qc = q / ER, qr = q % ER;
         const int qy = wrap_index(y0 - 1 + qr, ny, A.periodic[1]);
-        chunk(E + (qc * ER + qr) * EW + ROW, A.e_in + qc * N,
-              (qy >= 0 && mxa >= 0) ? qy * nx + mxa : -1, pe);
+        T *last = E + (qc * ER + qr) * EW + ROW;
+        const int off = (qy >= 0 && mxa >= 0) ? qy * nx + mxa : -1;
+        if (RAGGED) {  // its first place is all that is read
+          const bool in = off >= 0 && pe >= 0;
+          cp_async_value(last, in ? A.e_in + qc * N + pe + off : A.e_in, in);
+        } else {
+          chunk(last, A.e_in + qc * N, off, pe);
+        }
       }
     }
     if (H) {
       const long long ph = kh >= 0 ? (long long)kh * plane : -1;
 #pragma unroll
-      for (int c = 0; c < 3; c++) chunk(H + c * WARPS * ROW + hrow, A.h_in + c * N, off_h, ph);
+      for (int c = 0; c < 3; c++) {
+        if (RAGGED)
+          whole_row(H + (c * WARPS + w) * ROW, A.h_in + c * N, rowoff + x0 - VEC, my >= 0, ph);
+        else chunk(H + c * WARPS * ROW + hrow, A.h_in + c * N, off_h, ph);
+      }
       // the row's x-slab psi at plane kh, one value a lane of the slab's (xcoop reads them)
       if (xstage && kh >= 0) {
         T *xp = H + S::XP_OFF + w * S::XP;
@@ -1656,7 +1711,11 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
       if (w >= 1) {
         T *B = H + 3 * WARPS * ROW;
 #pragma unroll
-        for (int c = 0; c < 3; c++) chunk(B + c * RW * ROW + brow, A.cb + c * N, off_b, ph);
+        for (int c = 0; c < 3; c++) {
+          if (RAGGED)
+            whole_row(B + (c * RW + w - 1) * ROW, A.cb + c * N, rowoff + x0 - VEC, gy < ny, ph);
+          else chunk(B + c * RW * ROW + brow, A.cb + c * N, off_b, ph);
+        }
       }
     }
     cp_async_commit();
@@ -1741,7 +1800,9 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
 
   T hn[3][4], hprev[2][4];
   // prologue: H's new plane kbeg-1 (wrapped on a periodic z)
-  const int km = wrap_index(kbeg - 1, nz, A.periodic[2]);
+  // a grid one cell thick and periodic there is its own plane before: its new H serves (below)
+  const bool flat = nz == 1 && A.periodic[2];
+  const int km = flat ? -1 : wrap_index(kbeg - 1, nz, A.periodic[2]);
   // positions: E slots by position p = plane - kbeg + 1 (km at 0), HB slots alike
   issue(e_cur, km, hb_cur, km);                          // E(km), H(km), cb(km)
   issue(e_next, kbeg, nullptr, -1);                      // E(kbeg)
@@ -1806,7 +1867,7 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
   T fhz = A.fh[nx + ny + kbeg], fez = A.fe[nx + ny + kbeg];
   // the CPML's psi rows of this warp's row at plane kp into L2 (one thread a row): read from
   // memory a plane later, they then come from L2 rather than DRAM
-  const int pf0 = max(x0 - VEC, 0), pf1 = min(x0 + OWNX, nx);
+  const int pf0 = max(x0 - VEC, 0), pf1 = min(x0 + OWNX, A.pitch);
   auto prefetch_psi = [&](int kp) {
     const bool zsp = !A.periodic[2] && (kp < A.low[2] || kp >= nz - A.high[2]);
     const int zside = kp < A.low[2] ? 0 : 1;
@@ -1819,7 +1880,7 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
         for (int c = 0; c < 3; c += 2) {  // x and z along y
           const SlabEntry &sl = A.slab[f][c][1][sy];
           if (sl.count)
-            prefetch_l2(base + sl.psi + ((long long)kp * sl.count + (my - sl.from)) * nx + pf0, row);
+            prefetch_l2(base + sl.psi + ((long long)kp * sl.count + (my - sl.from)) * A.pitch + pf0, row);
         }
       }
       if (zsp) {
@@ -1827,8 +1888,7 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
         for (int c = 0; c < 2; c++) {  // x and y along z
           const SlabEntry &sl = A.slab[f][c][2][zside];
           if (sl.count)
-            prefetch_l2(base + sl.psi + (long long)(kp - sl.from) * plane + (long long)my * nx + pf0,
-                        row);
+            prefetch_l2(base + sl.psi + ((long long)(kp - sl.from) * ny + my) * A.pitch + pf0, row);
         }
       }
     }
@@ -1843,15 +1903,29 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
       if (lane == 0 && rowh && pf1 > pf0) prefetch_psi(k + 1);
     }
     compute_h(e_cur, e_next, hb_cur, k, fhz, true, hn);
+    if (flat) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        hprev[0][j] = hn[0][j];
+        hprev[1][j] = hn[1][j];
+      }
+    }
     // H's tile to memory, H_x and H_z to the row below
     const long long at = (long long)k * plane + rowoff + (mxb < 0 ? 0 : mxb);
     // the lossy form's ca of E's plane k, read now so that the barrier below covers the wait
     Vec4<T> ca[3];
     if (LOSSY && w >= 1 && any_own) {
 #pragma unroll
-      for (int c = 0; c < 3; c++) ca[c] = ld4(A.ca + c * N + at);
+      for (int c = 0; c < 3; c++) {
+        if (RAGGED) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) ca[c].v[j] = ownv[j] ? A.ca[c * N + at + j] : T(0);
+        } else {
+          ca[c] = ld4(A.ca + c * N + at);
+        }
+      }
     }
-    if (w >= 1 && lane >= 1 && rowh && mxb >= 0 && xb < nx) {
+    if (!RAGGED && w >= 1 && lane >= 1 && rowh && mxb >= 0 && xb < nx) {
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         Vec4<T> o;
@@ -1869,11 +1943,23 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
       }
       st4(sX + (size_t)w * ROW + VEC * lane, a);
       st4(sX + (size_t)(WARPS + w) * ROW + VEC * lane, b);
-      if (xco) {
+      if (xco || RAGGED) {
 #pragma unroll
         for (int j = 0; j < 4; j++) a.v[j] = hn[1][j];
         st4(sX + (size_t)(2 * WARPS + w) * ROW + VEC * lane, a);
       }
+    }
+    if (RAGGED && w >= 1 && rowh) {  // from the exchange rows, whole lines of the lanes' places
+      __syncwarp();
+      T *out = A.h_out + (long long)k * plane + rowoff + x0 - VEC + lane;
+      const T *row = sX + (size_t)w * ROW + lane;
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if ((inrow >> q & 1) && lane + 32 * q >= VEC) {
+          out[32 * q] = row[32 * q];
+          out[N + 32 * q] = row[2 * WARPS * ROW + 32 * q];
+          out[2 * N + 32 * q] = row[WARPS * ROW + 32 * q];
+        }
     }
     // the exchange row w goes to warp w+1 alone: a named barrier a pair of warps (id w+1, 64
     // threads; warp w arrives, warp w+1 waits) rather than the whole tile; warp w's own rows (its
@@ -1946,7 +2032,25 @@ __global__ void __launch_bounds__(quad::THREADS, 2) quad_kernel(StepArgs<T> A) {
                          const_cast<T *>(Hrow(hb_cur, 0)), WARPS * ROW, Brow(hb_cur, 0), RW * ROW,
                          lane, en);
       }
-      if (lane >= 1 && rowh && mxb >= 0 && xb < nx) {
+      if (RAGGED && rowh) {  // through the warp's rows of the old H
+        T *row = const_cast<T *>(Hrow(hb_cur, 0));
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          Vec4<T> o;
+#pragma unroll
+          for (int j = 0; j < 4; j++) o.v[j] = en[c][j];
+          st4(row + c * WARPS * ROW + VEC * lane, o);
+        }
+        __syncwarp();
+        T *out = A.e_out + (long long)k * plane + rowoff + x0 - VEC + lane;
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          if ((inrow >> q & 1) && lane + 32 * q >= VEC)
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+              out[c * N + 32 * q] = row[c * WARPS * ROW + lane + 32 * q];
+      } else if (lane >= 1 && rowh && mxb >= 0 && xb < nx) {
 #pragma unroll
         for (int c = 0; c < 3; c++) {
           Vec4<T> o;
@@ -2249,6 +2353,7 @@ struct DeviceSlab {
   int field, comp, axis;
   long long from, count, psi, coef, size;
   long long pf, pw;  // x slabs: the padded rows (see SlabEntry)
+  long long row, host_row, lead;  // a row's values here and in the host's array, and those before it
 };
 
 struct fdtd_ctx {
@@ -2256,6 +2361,7 @@ struct fdtd_ctx {
   int precision = 32;
   size_t elem = 4;
   int n[3];
+  int pitch = 0;  // n[0] padded to whole vectors of four: psi's rows along x (y and z slabs)
   long long N;
   int periodic[3], low[3], high[3];
   double dt;
@@ -2508,6 +2614,7 @@ StepArgs<T> step_args(fdtd_ctx *c) {
   StepArgs<T> A;
   for (int a = 0; a < 3; a++) {
     A.n[a] = c->n[a];
+    A.pitch = c->pitch;
     A.periodic[a] = c->periodic[a];
     A.low[a] = c->low[a];
     A.high[a] = c->high[a];
@@ -2572,8 +2679,13 @@ void launch_step(fdtd_ctx *c, const StepArgs<T> &A, bool ade = true) {
       kernel<<<grid, quad::THREADS, smem, c->stream>>>(A);
     };
     // media: the step (its E update without them), then their pass over the members
-    if (c->lossless) go(quad_kernel<T, false>);
-    else go(quad_kernel<T, true>);
+    if (c->n[0] % quad::VEC == 0) {
+      if (c->lossless) go(quad_kernel<T, false, false>);
+      else go(quad_kernel<T, true, false>);
+    } else {
+      if (c->lossless) go(quad_kernel<T, false, true>);
+      else go(quad_kernel<T, true, true>);
+    }
     if (c->media && ade)
       ade_kernel<T><<<(unsigned)((A.media.members + 255) / 256), 256, 0, c->stream>>>(A);
     return;
@@ -2901,7 +3013,7 @@ int bloch_impl(fdtd_ctx *a, fdtd_ctx *b, const std::vector<WrapDev> &hw,
       return fail(a, FDTD_E_STATE, "upload both parts' coefficients and fields before a run");
     if (c->naux_laid != c->naux + c->nbloch)
       return fail(a, FDTD_E_STATE, "set the sources again after the Bloch slots");
-    if (c->media && !c->quad)
+    if (c->media && (!c->quad || c->n[0] % quad::VEC != 0))
       return fail(a, FDTD_E_INVALID,
                   "Bloch sides with dispersive media step on grids whose nx is a multiple of 4");
   }
@@ -3100,6 +3212,7 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
     N *= c->n[a];
   }
   c->N = N;
+  c->pitch = (c->n[0] + 3) / 4 * 4;
   *out = c;
   if (!(dt > 0.0 && std::isfinite(dt)))
     return fail(c, FDTD_E_INVALID, "the time step must be positive, got %g", dt);
@@ -3136,7 +3249,11 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
     d.count = sl.count;
     d.pf = w == 0 ? sl.from / 4 * 4 : sl.from;
     d.pw = w == 0 ? (sl.from + sl.count + 3) / 4 * 4 - d.pf : sl.count;
-    d.size = d.pw * (N / c->n[w]);
+    // rows of whole vectors: along x the slab's places, along y and z the grid's rows, padded
+    d.row = w == 0 ? d.pw : c->pitch;
+    d.host_row = w == 0 ? sl.count : c->n[0];
+    d.lead = w == 0 ? sl.from - d.pf : 0;
+    d.size = d.row * (w == 0 ? N / c->n[0] : sl.count * (N / c->n[0] / c->n[w]));
     d.coef = (long long)coefs.size();
     // each slab's psi starts on a 16-element boundary, so a row of four values is one aligned
     // vector in f32 and two in f64
@@ -3186,10 +3303,11 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
   }
   {
     const char *force = getenv("PHOTONOXIDE_FDTD_KERNEL");
-    // the quad kernel takes four places along x at once: nx a multiple of 4, and no group of
-    // four holding places of both x CPMLs (an interior narrower than the group); its offsets
-    // within a plane are ints
-    const bool quad_ok = c->n[0] % 4 == 0 &&
+    // the quad kernel takes four places along x at once: nx a multiple of 4 or ends along x that
+    // don't wrap (a wrapped group of four would straddle two rows' ends), and no group of four
+    // holding places of both x CPMLs (an interior narrower than the group); its offsets within a
+    // plane are ints
+    const bool quad_ok = (c->n[0] % 4 == 0 || !c->periodic[0]) &&
         !(c->low[0] > 0 && c->high[0] > 0 && (c->low[0] - 1) / 4 == (c->n[0] - c->high[0]) / 4) &&
         (long long)c->n[0] * c->n[1] < (1LL << 31);
     std::string kind = force ? force : (quad_ok ? "quad" : "row");
@@ -3218,9 +3336,12 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
   // recompute fewer planes of H, and the two short interior runs (quad_runs), taken last, keep
   // the step's end short. On the 3D MMI (145 tiles) 7 runs timed best: 0.225 ms a step against
   // 0.228 with 9 or 10, 0.231 with 8, 0.239 with 6 and 0.243 with 13.
-  long long want = 6LL * sms;
+  // A run is four planes or more, but where even those leave SMs idle shorter ones, down to one
+  // plane: such a grid's step is as long as its longest CTA.
+  const long long slots = (long long)sms * (c->precision == 64 ? quad::ctas<double>() : quad::ctas<float>());
+  const long long want = 3 * slots;
   int chunks = (int)std::max<long long>(1, (want + tiles - 1) / tiles);
-  chunks = std::min(chunks, std::max(1, c->n[2] / 4));
+  chunks = std::min(chunks, (int)std::max<long long>(std::max(1, c->n[2] / 4), slots / tiles));
   const char *zc = getenv("PHOTONOXIDE_FDTD_ZCHUNKS");
   if (zc) chunks = std::max(1, atoi(zc));
   chunks = std::min(chunks, c->n[2]);
@@ -3283,13 +3404,13 @@ int fdtd_upload_fields(fdtd_ctx *c, const double *e, const double *h, const doub
     void *base = d.field == 1 ? c->psi_h[0] : c->psi_e;
     void *dst = (char *)base + d.psi * E;
     if (psi && psi[s]) {
-      if (d.axis == 0 && (d.pf != d.from || d.pw != d.count)) {
-        // the reference's rows of `count` values into the padded rows
-        long long rows = d.size / d.pw;
+      if (d.row != d.host_row) {
+        // the reference's rows into the padded rows
+        long long rows = d.size / d.row;
         std::vector<double> padded(d.size, 0.0);
         for (long long r = 0; r < rows; r++)
-          for (long long q = 0; q < d.count; q++)
-            padded[r * d.pw + (d.from - d.pf) + q] = psi[s][r * d.count + q];
+          for (long long q = 0; q < d.host_row; q++)
+            padded[r * d.row + d.lead + q] = psi[s][r * d.host_row + q];
         if (int r = upload(c, dst, padded.data(), d.size)) return r;
       } else if (int r = upload(c, dst, psi[s], d.size)) {
         return r;
@@ -3314,13 +3435,13 @@ int fdtd_download_fields(fdtd_ctx *c, double *e, double *h, double *const *psi) 
       const DeviceSlab &d = c->slabs[s];
       const void *base = d.field == 1 ? c->psi_h[c->parity] : c->psi_e;
       const void *src = (const char *)base + d.psi * c->elem;
-      if (d.axis == 0 && (d.pf != d.from || d.pw != d.count)) {
-        long long rows = d.size / d.pw;
+      if (d.row != d.host_row) {
+        long long rows = d.size / d.row;
         std::vector<double> padded(d.size);
         if (int r = download(c, padded.data(), src, d.size)) return r;
         for (long long r = 0; r < rows; r++)
-          for (long long q = 0; q < d.count; q++)
-            psi[s][r * d.count + q] = padded[r * d.pw + (d.from - d.pf) + q];
+          for (long long q = 0; q < d.host_row; q++)
+            psi[s][r * d.host_row + q] = padded[r * d.row + d.lead + q];
       } else if (int r = download(c, psi[s], src, d.size)) {
         return r;
       }
@@ -3996,6 +4117,7 @@ int fdtd_instance_view(fdtd_ctx *c, InstanceView *v) {
     v->step[a] = c->step[a];
   }
   v->N = c->N;
+  v->pitch = c->pitch;
   v->dt = c->dt;
   v->parity = c->parity;
   for (int p = 0; p < 2; p++) {
@@ -4065,7 +4187,7 @@ void fdtd_instance_advance(fdtd_ctx *c, long long steps) {
 }
 
 namespace {
-constexpr long long HOST_CHUNK = 1LL << 19;  // doubles: 4 MiB
+constexpr long long HOST_CHUNK = 1LL << 18;  // doubles: 2 MiB
 
 // n doubles of src added into the parts laid end to end, from place `at` of them on. Large runs
 // over the host's threads: one core adds at a fraction of what the link delivers.
@@ -4084,7 +4206,7 @@ void add_into_parts(const double *src, long long at, long long n, int nparts, do
 }
 }  // namespace
 
-// Read in 4 MiB chunks through two page-locked buffers, one filled while the other is added: a
+// Read in 2 MiB chunks through two page-locked buffers, one filled while the other is added: a
 // whole-plane transform (400 x 200, six components, 21 frequencies: 161 MB) had gone through three
 // pageable arrays made for each read, twice a call.
 int fdtd_instance_add_dft(fdtd_ctx *c, int nparts, double *const *parts, const long long *lens) {

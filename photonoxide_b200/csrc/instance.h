@@ -11,6 +11,7 @@
 struct InstanceView {
   int precision;
   int n[3];
+  int pitch;  // values from a row of a y slab's psi to the next (n[0] padded)
   long long N;
   int periodic[3], low[3], high[3];
   double dt, step[3];
