@@ -531,7 +531,7 @@ def _te_instances(count, seed=0, precision=32):
 def workload_batch(args):
     """Configuration 4, forward: 64 uneven 2D TE instances (sides log-uniform 256-1024 cells) with
     100x100 design regions, 6000 steps, batched (one persistent launch per step for all, CUDA-
-    graph chunks, tile shape by timing) against the same instances run one at a time: through the
+    graph chunks, tile shape by size) against the same instances run one at a time: through the
     3D engine (``one_at_a_time``) and as batches of one on the same TE kernel and tile shape
     (``one_at_a_time_te_kernel``, which isolates the batching's own gain)."""
     from photonoxide_b200.batch import Batch
@@ -539,7 +539,7 @@ def workload_batch(args):
     sims = _te_instances(64)
     cells = sum(s.grid.cells() for s in sims)
     B = Batch(sims)
-    B.run(480)  # the tile shape's trial chunks
+    B.run(480)  # warm-up
     _, tb = _timed(lambda: B.run(steps))
     alone = _te_instances(64)
     for s in alone:

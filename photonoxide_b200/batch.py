@@ -1,5 +1,5 @@
 """Batched 2D TE simulations: several :class:`~photonoxide_b200.fdtd.Simulation` grids stepped
-together on the GPU, one persistent launch per step for all of them (include/photonoxide_batch.h).
+together on the GPU, a launch taking several steps of all of them (include/photonoxide_batch.h).
 
 Each simulation keeps its own setup, sources and monitors; after ``Batch.run(n)`` it reads out
 (fields, probes, transforms, fluxes) exactly as if ``Simulation.run(n)`` had taken the steps,
@@ -70,9 +70,10 @@ class Batch:
         raise GpuError(msg)
 
     def run(self, steps: int) -> "Batch":
-        """``steps`` steps of every simulation. The first run of a batch without a fixed tile
-        shape (32x8, 32x16, 64x4, 64x8, 128x2, 128x4 or the 124x7 rows) times each shape on
-        chunks of these steps and keeps the fastest, when it has at least 480 of them."""
+        """``steps`` steps of every simulation. A batch without a fixed tile shape takes tiles of
+        several steps a launch: 112x16 (eight steps) for few cells, 120x40 (f32) or 120x24 (f64)
+        (four) for many. The shapes of one step a launch are 32x8, 32x16, 64x4, 64x8, 128x2, 128x4
+        and the 124x7 rows."""
         self._check(_lib().pxs_batch_run(self._h, int(steps)))
         return self
 

@@ -10,20 +10,21 @@
 // kernel (curl, the CPML slabs along x then y, then the sources), so a simulation stepped in a
 // batch has the bits it has stepped alone.
 //
-// One step is ONE persistent launch: CTAs (a few per SM) take tiles of TW x TH cells from the
-// list of all the grids' tiles. A tile computes H_z over itself and the row and column below it
-// (its neighbours compute the same values), adds the magnetic sources there, then updates E_x and
-// E_y on its cells, adds the electric sources, and writes both to the other copy of the fields.
+// A launch takes several steps of all the grids (te_block.cuh): a CTA holds a tile and a halo of as
+// many places around it as the steps it takes. With a tile shape of one step (fdtd_batch_set_tile) a
+// step is one persistent launch: CTAs (a few per SM) take tiles of TW x TH cells from the list of all
+// the grids' tiles; a tile computes H_z over itself and the row and column below it (its neighbours
+// compute the same values), adds the magnetic sources there, then updates E_x and E_y on its cells,
+// adds the electric sources, and writes both to the other copy of the fields.
 // Steps run in chunks of G: the source waveforms and transform phases of a chunk are evaluated
-// first (f64, the reference's exp and sincos), the chunk's step launches follow, each with a
-// launch that copies the monitored values into a ring; at the chunk's end one launch adds the
-// ring into the f64 transform sums in time order. A chunk is captured
-// once as a CUDA graph and replayed. The tile shape is chosen by timing: the first run tries each
-// shape on a chunk of real steps (every shape gives the same bits) and keeps the fastest.
+// first (f64, the reference's exp and sincos), the chunk's step launches follow, the monitored
+// values copied into a ring as they go; at the chunk's end one launch adds the ring into the f64
+// transform sums in time order. A chunk is captured once as a CUDA graph and replayed.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -54,6 +55,8 @@ struct TeInst {
   double dt64;
   T *e[2], *h[2], *psi_h[2];
   T *psi_e;
+  T *psi_e2;           // te_block_kernel's other copy of E's psi, and which is current
+  int psi_parity;
   const T *ca, *cb, *fe, *fh, *coefs;
   // the CPML slabs a TE grid has: H_z along x and y, E_y along x, E_x along y (per side)
   SlabEntry hx[2], hy[2], ex[2], ey[2];
@@ -584,15 +587,40 @@ __global__ void te_contract_kernel(const TeInst<T> *insts, const RecItem *items,
                      s.volume, s.nf - f0);
 }
 
-// After `count` steps: each instance's step index, copy and record row move on.
+// After `count` steps: each instance's step index, current copies (`flips` times the fields',
+// `psi_flips` times E's psi's) and record row move on.
 template <typename T>
-__global__ void te_advance_kernel(TeInst<T> *insts, int n, int count) {
+__global__ void te_advance_kernel(TeInst<T> *insts, int n, int count, int flips, int psi_flips) {
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   TeInst<T> &I = insts[q];
   I.first += count;
-  I.parity = (I.parity + count) & 1;
+  I.parity = (I.parity + flips) & 1;
+  I.psi_parity = (I.psi_parity + psi_flips) & 1;
   if (I.rows) I.rows += (long long)count * I.nprobes;
+}
+
+// Where instance 0's next run starts: its step index, current copies and record row.
+template <typename T>
+__global__ void te_start_kernel(TeInst<T> *insts, long long first, int parity, double *rows) {
+  insts[0].first = first;
+  insts[0].parity = parity;
+  insts[0].psi_parity = 0;
+  insts[0].rows = rows;
+}
+
+// Ranges of values that are all zero while a 2D grid's run is TE: a nonzero one sets *bad.
+struct ZeroRanges {
+  const void *at[16];
+  long long len[16];
+  int count;
+};
+template <typename T>
+__global__ void te_zero_kernel(ZeroRanges R, int *bad) {
+  const T *p = (const T *)R.at[blockIdx.y];
+  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < R.len[blockIdx.y];
+       q += (long long)gridDim.x * blockDim.x)
+    if (p[q] != T(0)) atomicOr(bad, 1);
 }
 
 // Nonzero values among H_x, H_y, E_z of the current copy (the batch steps TE grids only).
@@ -659,7 +687,7 @@ __device__ __forceinline__ T coef_a(const TeInst<T> &I, const SlabEntry &s, int 
 
 template <typename T, int TW, int TH>
 __global__ void __launch_bounds__(THREADS) te_adjoint_kernel(const TeInst<T> *insts,
-                                                             AdjState<T> A, int ntiles) {
+                                                             AdjState<T> A, int tiles_x, int ntiles) {
   constexpr int HW = TW + 1, HH = TH + 1;
   __shared__ T sh[HW * HH];  // H~ of the step's H_z over the tile and the row and column below
   const TeInst<T> &I = insts[0];
@@ -689,7 +717,7 @@ __global__ void __launch_bounds__(THREADS) te_adjoint_kernel(const TeInst<T> *in
     return phi[s.psi + (long long)(y - s.from) * I.pitch + x] + I.dt * hbar;
   };
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int x0 = (t % I.tiles_x) * TW, y0 = (t / I.tiles_x) * TH;
+    const int x0 = (t % tiles_x) * TW, y0 = (t / tiles_x) * TH;
     // -- H~ of the step's new H_z (total)
     for (int q = threadIdx.x; q < HW * HH; q += THREADS) {
       const int lx = q % HW, ly = q / HW;
@@ -860,15 +888,27 @@ __global__ void te_grad_kernel(const long long *design, long long n, const T *K,
   grad[d] += (double)A.e[A.cur][design[d]] * (double)K[d];
 }
 
+}  // namespace pxb
+
+#include "te_block.cuh"
+
+namespace pxb {
+
 struct Shape {
   int tw, th;
+  int halo;  // te_block_kernel's: the steps a launch takes at most; 0: the kernels of one step
 };
-// the last: te_quad_kernel's rows
-const Shape SHAPES[] = {{32, 8}, {32, 16}, {64, 4}, {64, 8}, {128, 2}, {128, 4},
-                        {teq::OWN, teq::RW}};
-constexpr int QUAD_SHAPE = 6;
+// the seventh: te_quad_kernel's rows; the last three: te_block_kernel's (120 x 24 in f64, where the
+// taller tile's values have no registers, 120 x 40 in f32)
+const Shape SHAPES[] = {{32, 8, 0}, {32, 16, 0}, {64, 4, 0}, {64, 8, 0}, {128, 2, 0}, {128, 4, 0},
+                        {teq::OWN, teq::RW, 0}, {112, 16, 8}, {120, 24, 4}, {120, 40, 4}};
+constexpr int QUAD_SHAPE = 6, BLOCK_SMALL = 7, BLOCK_LARGE = 8, BLOCK_TALL = 9;
 constexpr int NSHAPES = sizeof(SHAPES) / sizeof(SHAPES[0]);
-constexpr int DEFAULT_SHAPE = 3;  // 64 x 8
+// te_block_kernel's warps: f32, 16 of 2 rows (eight steps a launch) or 3 (four: fewer halo places);
+// f64, 8 of 4 rows.
+template <typename T>
+constexpr int BLOCK_WARPS = sizeof(T) == 4 ? 16 : 8;
+static_assert(G % 16 == 0, "a chunk is an even number of launches of up to 8 steps");
 
 }  // namespace pxb
 
@@ -880,7 +920,7 @@ struct fdtd_batch {
   int precision = 32;
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr, t0 = nullptr, t1 = nullptr;
-  int shape = -1;  // index into SHAPES; -1: choose by timing on the next run
+  int shape = -1;  // index into SHAPES; -1: by the size on the next run (block_shape)
   long long launches = 0;
   int sms = 148;
   std::vector<void *> allocs;  // this run's tables
@@ -890,6 +930,12 @@ struct fdtd_batch {
   int ntiles = 0;
   int *d_tile_inst = nullptr;
   int *d_hbucket = nullptr, *d_ebucket = nullptr;
+  // te_block_kernel's: the recorded and design values by tile
+  int *d_hrecs = nullptr, *d_erecs = nullptr, *d_dbucket = nullptr;
+  TeRec *d_hrec = nullptr, *d_erec = nullptr;
+  TeDesign *d_design_items = nullptr;
+  int psi_flips = 0;  // E's psi's current copy: odd, the second
+  std::vector<void *> psi2;  // the second copies, by instance
   Group *d_hgroups = nullptr, *d_egroups = nullptr;
   Entry *d_entries = nullptr;
   Wave *d_waves = nullptr;
@@ -909,12 +955,16 @@ struct fdtd_batch {
   // at the design's values into K[step - k_first][value]
   bool record = true;
   const long long *d_design = nullptr;
+  const std::vector<long long> *design = nullptr;  // the same on the host
   long long ndesign = 0;
   void *d_K = nullptr;
   long long k_first = 0;
   // the tables and graph stay good for the next run while every member is as the last run left
   // it: the same generation (no engine call since), step index and current copy
   bool reusable = false;
+  // a context's own batch of one, on its stream (fdtd_solo_run); aux: it has a plane wave's run
+  bool solo = false, aux = false;
+  unsigned long long solo_layout = 0;
   bool cap_record = true;
   long long per_chunk = 0;  // the graph's kernels
   std::vector<unsigned long long> gens;
@@ -994,7 +1044,13 @@ template <typename T>
 int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vector<int64_t> &first,
           const std::vector<int> &parity, const std::vector<double *> &rows, int sh) {
   free_tables(b);
-  const int TW = SHAPES[sh].tw, TH = SHAPES[sh].th;
+  const int TW = SHAPES[sh].tw, TH = SHAPES[sh].th, halo = SHAPES[sh].halo;
+  const int bh = TH + 2 * halo;  // a region's rows (te_block_kernel)
+  std::vector<int> hrb{0}, erb{0}, db{0};
+  std::vector<TeRec> hrec, erec;
+  std::vector<TeDesign> ditems;
+  b->psi2.assign(views.size(), nullptr);
+  b->psi_flips = 0;
   std::vector<TeInst<T>> insts(views.size());
   std::vector<int> tile_inst;
   std::vector<int> hb{0}, eb{0};
@@ -1056,7 +1112,8 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
     I.wave0 = (int)waves.size();
     I.nwaves = (int)v.waves->size();
     std::vector<int> pt(I.nwaves, 0);
-    for (const fdtd_injection &x : *v.inj) pt[x.emitter] = x.point ? 1 : 0;
+    for (const fdtd_injection &x : *v.inj)
+      if (x.point != 2) pt[x.emitter] = x.point ? 1 : 0;
     for (int e = 0; e < I.nwaves; e++) {
       Wave w;
       w.kind = (*v.waves)[e].kind;
@@ -1074,6 +1131,8 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
       std::vector<std::vector<Entry>> lists;
       for (const fdtd_injection &x : *v.inj) {
         if (x.field != f) continue;
+        // a plane wave's couplings of the components that stay zero (solo_ok) take nothing
+        if (x.point == 2 && (f == 1) != (x.component == 2)) continue;
         const long long place = (long long)x.component * v.N + x.r;
         auto it = index.find(place);
         int at;
@@ -1088,8 +1147,8 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
         Entry en;
         en.are = x.a_re;
         en.aim = x.a_im;
-        en.emitter = I.wave0 + x.emitter;
-        en.pad = 0;
+        en.emitter = I.wave0 + (x.point == 2 ? I.nwaves : 0) + x.emitter;
+        en.pad = x.point == 2 ? 1 : 0;
         lists[at].push_back(en);
       }
       for (size_t g = 0; g < places.size(); g++) {
@@ -1109,6 +1168,29 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
           for (const Entry &e : lists[g]) entries.push_back(e);
           to.push_back(c);
         };
+        if (halo > 0) {
+          // every place of every region that holds the value, wrapped images included
+          std::vector<std::pair<int, int>> px, py;
+          auto images = [&](int c, int n, int w, int len, int tiles, int periodic,
+                            std::vector<std::pair<int, int>> &out) {
+            for (int t = 0; t < tiles; t++) {
+              const int lo = t * w - halo;  // the region's first place
+              if (!periodic) {
+                if (c >= lo && c < lo + len) out.push_back({t, c - lo});
+                continue;
+              }
+              int first = (c - lo) % n;
+              if (first < 0) first += n;
+              for (int q = first; q < len; q += n) out.push_back({t, q});
+            }
+          };
+          images(x, I.nx, TW, BW, I.tiles_x, I.px, px);
+          images(y, I.ny, TH, bh, tiles_y, I.py, py);
+          for (auto oy : py)
+            for (auto ox : px)
+              add((f ? hper : eper)[oy.first * I.tiles_x + ox.first], oy.second * BW + ox.second);
+          continue;
+        }
         if (f == 0) {
           const int tx = x / TW, ty = y / TH;
           add(eper[ty * I.tiles_x + tx], (y - ty * TH) * TW + (x - tx * TW));
@@ -1150,13 +1232,69 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
     I.nslots = v.nvalues > 0 ? v.nslots : 0;
     for (int s = 0; s < I.nslots; s++) slot_items.push_back(make_int2((int)i, s));
     slots += I.nslots;
-    for (long long q = 0; q < v.nvalues; q++) rec.push_back(RecItem{(int)i, 0, q, nring++});
-    for (int p = 0; p < v.nprobes; p++) rec.push_back(RecItem{(int)i, 1, p, -1});
+    if (halo == 0) {
+      for (long long q = 0; q < v.nvalues; q++) rec.push_back(RecItem{(int)i, 0, q, nring++});
+      for (int p = 0; p < v.nprobes; p++) rec.push_back(RecItem{(int)i, 1, p, -1});
+    } else {
+      // the recorded and the design's values by tile, each in the tile that owns its place
+      const size_t E = sizeof(T);
+      void *second = nullptr;
+      BTRY(b, cudaMallocAsync(&second, std::max<size_t>(v.psi_e_len, 1) * E, b->stream));
+      b->allocs.push_back(second);
+      b->psi2[i] = second;
+      I.psi_e2 = (T *)second;
+      std::vector<std::vector<TeRec>> hp(ntile), ep(ntile);
+      std::vector<std::vector<TeDesign>> dp(ntile);
+      auto home = [&](long long r, int *local) {
+        const int x = (int)(r % I.nx), y = (int)(r / I.nx), tx = x / TW, ty = y / TH;
+        *local = (y - ty * TH + halo) * BW + (x - tx * TW + halo);
+        return ty * I.tiles_x + tx;
+      };
+      auto take = [&](long long place, long long col, int probe) {
+        const bool hf = (place >> 62) != 0;
+        const long long p = place & ((1LL << 62) - 1);
+        const int comp = (int)(p / v.N);
+        TeRec it{0, hf ? (comp == 2 ? 2 : 3) : (comp < 2 ? comp : 3), col, probe, 0};
+        if (it.comp == 3 && col >= 0) return;  // zero all along, and so is its sum
+        const int t = home(p % v.N, &it.local);
+        (it.comp == 2 ? hp : ep)[t].push_back(it);
+      };
+      if (b->record) {
+        std::vector<long long> where(v.nvalues), probes(v.nprobes);
+        if (v.nvalues)
+          BTRY(b, cudaMemcpyAsync(where.data(), v.where, v.nvalues * 8, cudaMemcpyDeviceToHost, b->stream));
+        if (v.nprobes)
+          BTRY(b, cudaMemcpyAsync(probes.data(), v.probes, v.nprobes * 8, cudaMemcpyDeviceToHost, b->stream));
+        BTRY(b, cudaStreamSynchronize(b->stream));
+        for (long long q = 0; q < v.nvalues; q++) {
+          const int comp = (int)((where[q] & ((1LL << 62) - 1)) / v.N);
+          if ((where[q] >> 62 != 0) != (comp == 2)) continue;
+          rec.push_back(RecItem{(int)i, 0, q, nring});
+          take(where[q], nring++, 0);
+        }
+        for (int p = 0; p < v.nprobes; p++) take(probes[p], -1, p);
+      }
+      if (i == 0 && b->ndesign > 0 && b->design)
+        for (long long d = 0; d < b->ndesign; d++) {
+          const long long place = (*b->design)[d];
+          TeDesign it{0, (int)(place / v.N), d};
+          const int t = home(place % v.N, &it.local);
+          dp[t].push_back(it);
+        }
+      for (int t = 0; t < ntile; t++) {
+        hrec.insert(hrec.end(), hp[t].begin(), hp[t].end());
+        erec.insert(erec.end(), ep[t].begin(), ep[t].end());
+        ditems.insert(ditems.end(), dp[t].begin(), dp[t].end());
+        hrb.push_back((int)hrec.size());
+        erb.push_back((int)erec.size());
+        db.push_back((int)ditems.size());
+      }
+    }
   }
   b->ntiles = (int)tile_inst.size();
   b->freq_chunks = 1;
   for (const InstanceView &v : views) b->freq_chunks = std::max(b->freq_chunks, v.freq_chunks);
-  b->nwaves_total = (int)waves.size();
+  b->nwaves_total = (int)waves.size() + (views.size() == 1 ? views[0].naux : 0);
   b->nslots_total = slots;
   b->nwave_items = (int)wave_items.size();
   b->nslot_items = (int)slot_items.size();
@@ -1173,6 +1311,17 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
   if (int r = upload_vec(b, &b->d_wave_items, wave_items)) return r;
   if (int r = upload_vec(b, &b->d_slot_items, slot_items)) return r;
   if (int r = upload_vec(b, &b->d_rec, rec)) return r;
+  b->d_dbucket = nullptr;
+  if (halo > 0) {
+    if (int r = upload_vec(b, &b->d_hrecs, hrb)) return r;
+    if (int r = upload_vec(b, &b->d_erecs, erb)) return r;
+    if (int r = upload_vec(b, &b->d_hrec, hrec)) return r;
+    if (int r = upload_vec(b, &b->d_erec, erec)) return r;
+    if (!ditems.empty()) {
+      if (int r = upload_vec(b, &b->d_dbucket, db)) return r;
+      if (int r = upload_vec(b, &b->d_design_items, ditems)) return r;
+    }
+  }
   if (int r = zeros(b, &b->d_waves_h, (size_t)G * std::max(b->nwaves_total, 1) * 2)) return r;
   if (int r = zeros(b, &b->d_waves_e, (size_t)G * std::max(b->nwaves_total, 1) * 2)) return r;
   if (int r = zeros(b, &b->d_phase, (size_t)G * std::max(b->nslots_total, 1) * 2)) return r;
@@ -1193,6 +1342,50 @@ void launch_step(fdtd_batch *b, int m) {
       (const TeInst<T> *)b->d_insts, b->d_tile_inst, b->ntiles, b->d_hbucket, b->d_ebucket,
       b->d_hgroups, b->d_egroups, b->d_entries,
       b->d_waves_h + 2LL * m * b->nwaves_total, b->d_waves_e + 2LL * m * b->nwaves_total, m);
+}
+
+// te_block_kernel: `count` steps from step m of the chunk, the chunk's launch number `launch`;
+// with no steps, only its attributes are set.
+template <typename T, int HALO, int ROWS>
+void launch_block(fdtd_batch *b, int m, int count, int launch) {
+  constexpr int NW = BLOCK_WARPS<T>, R = ROWS / NW;
+  auto kernel = te_block_kernel<T, NW, R, HALO>;
+  constexpr size_t smem = block_smem_values<T, NW, R>() * sizeof(T);
+  static_assert(smem <= 227 * 1024, "a CTA's shared memory");
+  if (count == 0) {  // before the first launch: a captured one takes no attribute
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return;
+  }
+  BlockArgs<T> A;
+  A.hbucket = b->d_hbucket;
+  A.ebucket = b->d_ebucket;
+  A.hgroups = b->d_hgroups;
+  A.egroups = b->d_egroups;
+  A.entries = b->d_entries;
+  A.waves_h = b->d_waves_h;
+  A.waves_e = b->d_waves_e;
+  A.nwaves = b->nwaves_total;
+  A.hrecs = b->d_hrecs;
+  A.erecs = b->d_erecs;
+  A.hrec = b->d_hrec;
+  A.erec = b->d_erec;
+  A.ring = (T *)b->d_ring;
+  A.nring = b->nring;
+  A.dbucket = b->ndesign > 0 ? b->d_dbucket : nullptr;
+  A.design = b->d_design_items;
+  A.K = (T *)b->d_K;
+  A.k_first = b->k_first;
+  A.ndesign = b->ndesign;
+  A.record = b->record ? 1 : 0;
+  kernel<<<b->ntiles, NW * 32, smem, b->stream>>>((const TeInst<T> *)b->d_insts, b->d_tile_inst, A, m,
+                                                  count, launch);
+}
+
+template <typename T>
+void launch_shape(fdtd_batch *b, int m, int count, int launch) {
+  if (b->shape == BLOCK_SMALL) launch_block<T, 8, 32>(b, m, count, launch);
+  else if (sizeof(T) == 4) launch_block<float, 4, 48>(b, m, count, launch);
+  else launch_block<double, 4, 32>(b, m, count, launch);
 }
 
 template <typename T>
@@ -1229,10 +1422,15 @@ int occupancy(fdtd_batch *b) {
 }
 
 // `count` (<= G) steps of the current tables on the batch's stream; then the instances advance.
+// Returns how often the current copy has changed.
 template <typename T>
-void enqueue(fdtd_batch *b, int count) {
+int enqueue(fdtd_batch *b, int count) {
   TeInst<T> *insts = (TeInst<T> *)b->d_insts;
   const int n = (int)b->ctxs.size();
+  if (b->aux)  // a plane wave's auxiliary run, its incident values after the emitters' (solo)
+    b->launches += fdtd_instance_aux(
+        b->ctxs[0], b->nwaves_total, (const long long *)((char *)b->d_insts + offsetof(TeInst<T>, first)),
+        count, b->d_waves_h, b->d_waves_e);
   if (b->nwave_items > 0) {
     int total = b->nwave_items * G;
     te_waves_kernel<T><<<(total + 127) / 128, 128, 0, b->stream>>>(
@@ -1246,7 +1444,17 @@ void enqueue(fdtd_batch *b, int count) {
         insts, b->d_slot_items, b->nslot_items, b->nslots_total, b->d_phase);
     b->launches++;
   }
-  for (int m = 0; m < count; m++) {
+  const int halo = SHAPES[b->shape].halo;
+  int flips = count, psi_flips = 0;
+  if (halo > 0) {
+    flips = 0;
+    for (int m = 0; m < count; m += halo, flips++) {
+      launch_shape<T>(b, m, std::min(halo, count - m), flips);
+      b->launches++;
+    }
+    psi_flips = flips;
+  }
+  for (int m = 0; m < count && halo == 0; m++) {
     step_by_shape<T>(b, m);
     b->launches++;
     if (b->nrec > 0 && b->record) {
@@ -1267,15 +1475,18 @@ void enqueue(fdtd_batch *b, int count) {
         count);
     b->launches++;
   }
-  te_advance_kernel<T><<<(n + 127) / 128, 128, 0, b->stream>>>(insts, n, count);
+  te_advance_kernel<T><<<(n + 127) / 128, 128, 0, b->stream>>>(insts, n, count, flips, psi_flips);
   b->launches++;
+  return flips;
 }
 
 // The run's steps from `done` on with the current tables: whole chunks by the captured graph
 // (captured now if there is none), the rest launched; then the members' streams wait for them.
 template <typename T>
-int finish_run(fdtd_batch *b, int64_t steps, int64_t done, const std::vector<InstanceView> &views) {
+int finish_run(fdtd_batch *b, int64_t steps, const std::vector<InstanceView> &views, int *flips) {
   const int n = (int)b->ctxs.size();
+  int64_t done = 0;
+  *flips = 0;  // whole chunks are an even number of changes
   const int64_t full = (steps - done) / G;
   if (full > 0) {
     if (!b->graph) {
@@ -1300,16 +1511,37 @@ int finish_run(fdtd_batch *b, int64_t steps, int64_t done, const std::vector<Ins
     }
     done += full * G;
   }
-  if (done < steps) enqueue<T>(b, (int)(steps - done));
+  if (done < steps) *flips = enqueue<T>(b, (int)(steps - done));
   BTRY(b, cudaGetLastError());
-  BTRY(b, cudaEventRecord(b->done, b->stream));
+  if (SHAPES[b->shape].halo > 0) {
+    // E's psi ends where the engine keeps it
+    b->psi_flips = (b->psi_flips + *flips) & 1;
+    if (b->psi_flips)
+      for (int i = 0; i < n; i++)
+        if (views[i].psi_e_len > 0)
+          BTRY(b, cudaMemcpyAsync(views[i].psi_e, b->psi2[i], views[i].psi_e_len * sizeof(T),
+                                  cudaMemcpyDeviceToDevice, b->stream));
+  }
+  if (!b->solo) BTRY(b, cudaEventRecord(b->done, b->stream));
   for (int i = 0; i < n; i++) {
-    BTRY(b, cudaStreamWaitEvent(views[i].stream, b->done, 0));
-    fdtd_instance_advance(b->ctxs[i], steps);
+    if (!b->solo) BTRY(b, cudaStreamWaitEvent(views[i].stream, b->done, 0));
+    fdtd_instance_advance(b->ctxs[i], steps, *flips);
   }
   // no wait here: each context's stream waits for the batch's work (the event), so its later
   // calls see the steps; the batch's next run orders after them on the batch's stream
   return 0;
+}
+
+// The tile shape of a batch whose caller fixed none: te_block_kernel's, eight steps a launch while
+// its tiles fill the SMs a few times over, four steps beyond (us a step, eight against four, f32: one
+// 537 x 541 grid 6.6 and 9.8; 1.29 M cells in six 17.8 and 18.3; 2.6 M in twelve 33.7 and 32.4; 19.2 M
+// in 64 217 and 195; one step a launch 12.2, 29.9, 54.3 and 373).
+int block_shape(const std::vector<InstanceView> &views, int sms) {
+  long long tiles = 0;
+  for (const InstanceView &v : views)
+    tiles += (long long)((v.n[0] + SHAPES[BLOCK_SMALL].tw - 1) / SHAPES[BLOCK_SMALL].tw) *
+             ((v.n[1] + SHAPES[BLOCK_SMALL].th - 1) / SHAPES[BLOCK_SMALL].th);
+  return tiles <= 6LL * sms ? BLOCK_SMALL : views[0].precision == 64 ? BLOCK_LARGE : BLOCK_TALL;
 }
 
 // A run whose members are all as the last run left them: its tables and graph serve again, the
@@ -1337,10 +1569,11 @@ int run_again(fdtd_batch *b, int64_t steps, const int64_t *first_steps, bool *ra
     BTRY(b, cudaEventRecord(b->member_ev[i], views[i].stream));
     BTRY(b, cudaStreamWaitEvent(b->stream, b->member_ev[i], 0));
   }
-  if (int r = finish_run<T>(b, steps, 0, views)) return r;
+  int flips = 0;
+  if (int r = finish_run<T>(b, steps, views, &flips)) return r;
   for (int i = 0; i < n; i++) {
     b->next_first[i] += steps;
-    b->next_parity[i] = (int)((b->next_parity[i] + steps) & 1);
+    b->next_parity[i] = (b->next_parity[i] + flips) & 1;
   }
   *ran = true;
   return 0;
@@ -1405,54 +1638,13 @@ int run_impl(fdtd_batch *b, int64_t steps, const int64_t *first_steps) {
         return bfail(b, FDTD_E_INVALID,
                      "simulation %d has H_x, H_y or E_z values: the batch steps TE fields only", i);
   }
-  // where the device's descriptors have moved the instances to
-  auto pull = [&]() -> int {
-    std::vector<TeInst<T>> now(n);
-    BTRY(b, cudaStreamSynchronize(b->stream));
-    BTRY(b, cudaMemcpy(now.data(), b->d_insts, n * sizeof(TeInst<T>), cudaMemcpyDeviceToHost));
-    for (int i = 0; i < n; i++) {
-      first[i] = now[i].first;
-      parity[i] = now[i].parity;
-      rows[i] = now[i].rows;
-    }
-    return 0;
-  };
-  auto rebuild = [&](int sh) -> int {
-    if (int r = build<T>(b, views, first, parity, rows, sh)) return r;
-    b->blocks = occupancy<T>(b) * b->sms;
-    return 0;
-  };
-  int64_t done = 0;
-  // the tile shape: each shape times one chunk of real steps (after one warm chunk), the
-  // fastest is kept; every shape gives the same bits
-  if (b->shape < 0) {
-    if (steps >= 2LL * NSHAPES * G + G) {
-      float best = 1e30f;
-      int pick = 0;
-      for (int sh = 0; sh < NSHAPES; sh++) {
-        if (int r = rebuild(sh)) return r;
-        enqueue<T>(b, G);
-        BTRY(b, cudaEventRecord(b->t0, b->stream));
-        enqueue<T>(b, G);
-        BTRY(b, cudaEventRecord(b->t1, b->stream));
-        BTRY(b, cudaEventSynchronize(b->t1));
-        float ms = 0.f;
-        BTRY(b, cudaEventElapsedTime(&ms, b->t0, b->t1));
-        if (ms < best) {
-          best = ms;
-          pick = sh;
-        }
-        done += 2 * G;
-        if (int r = pull()) return r;
-      }
-      b->shape = pick;
-    } else {
-      b->shape = DEFAULT_SHAPE;
-    }
-  }
-  if (int r = rebuild(b->shape)) return r;
+  if (b->shape < 0) b->shape = block_shape(views, b->sms);
+  if (int r = build<T>(b, views, first, parity, rows, b->shape)) return r;
+  if (SHAPES[b->shape].halo > 0) launch_shape<T>(b, 0, 0, 0);
+  else b->blocks = occupancy<T>(b) * b->sms;
   b->reusable = false;
-  if (int r = finish_run<T>(b, steps, done, views)) return r;
+  int flips = 0;
+  if (int r = finish_run<T>(b, steps, views, &flips)) return r;
   b->reusable = true;
   b->cap_record = b->record;
   b->gens.assign(n, 0);
@@ -1461,12 +1653,93 @@ int run_impl(fdtd_batch *b, int64_t steps, const int64_t *first_steps) {
   for (int i = 0; i < n; i++) {
     b->gens[i] = views[i].generation;
     b->next_first[i] = (first_steps ? first_steps[i] : 0) + steps;
-    b->next_parity[i] = (int)((views[i].parity + steps) & 1);
+    b->next_parity[i] = (views[i].parity + flips) & 1;
   }
   return 0;
 }
 
+// A context's own run on the TE tiles (fdtd_solo_run).
+template <typename T>
+int solo_run(fdtd_batch *b, bool check, int64_t steps, int64_t first, bool *te) {
+  std::vector<InstanceView> views(1);
+  InstanceView &v = views[0];
+  if (int r = fdtd_instance_view(b->ctxs[0], &v)) return r;
+  const size_t E = sizeof(T);
+  *te = false;
+  if (check) {
+    // H_x, H_y and E_z, and their psi, all zero; then the other copies' fields are too
+    ZeroRanges R;
+    R.count = 0;
+    auto add = [&](const void *at, long long len) {
+      if (len > 0 && R.count < 16) R.at[R.count] = at, R.len[R.count] = len, R.count++;
+    };
+    add(v.h[v.parity], 2 * v.N);
+    add((const char *)v.e[v.parity] + 2 * v.N * E, v.N);
+    for (int f = 0; f < 2; f++)
+      for (int c = 0; c < 3; c++) {
+        if ((f == 1) == (c == 2)) continue;
+        for (int a = 0; a < 2; a++)
+          for (int side = 0; side < 2; side++) {
+            const SlabEntry &s = v.table[f][c][a][side];
+            if (s.count == 0) continue;
+            add((const char *)(f == 1 ? v.psi_h[v.parity] : v.psi_e) + s.psi * E,
+                a == 0 ? (long long)s.pw * v.n[1] : (long long)s.count * v.pitch);
+          }
+      }
+    if (!b->d_flags) BTRY(b, cudaMallocAsync(&b->d_flags, 4, b->stream));
+    int bad = 0;
+    BTRY(b, cudaMemsetAsync(b->d_flags, 0, 4, b->stream));
+    te_zero_kernel<T><<<dim3(64, R.count), 256, 0, b->stream>>>(R, b->d_flags);
+    BTRY(b, cudaGetLastError());
+    BTRY(b, cudaMemcpyAsync(&bad, b->d_flags, 4, cudaMemcpyDeviceToHost, b->stream));
+    BTRY(b, cudaStreamSynchronize(b->stream));
+    if (bad) return 0;
+    BTRY(b, cudaMemsetAsync(v.h[1 - v.parity], 0, 2 * v.N * E, b->stream));
+    BTRY(b, cudaMemsetAsync((char *)v.e[1 - v.parity] + 2 * v.N * E, 0, v.N * E, b->stream));
+  }
+  double *rows = nullptr;
+  if (int r = fdtd_instance_reserve(b->ctxs[0], steps, &rows)) return r;
+  if (!b->reusable || b->solo_layout != v.layout) {
+    b->reusable = false;
+    b->aux = v.naux > 0;
+    b->shape = block_shape(views, b->sms);
+    if (int r = build<T>(b, views, {first}, {v.parity}, {rows}, b->shape)) return r;
+    launch_shape<T>(b, 0, 0, 0);
+    b->solo_layout = v.layout;
+    b->reusable = true;
+  }
+  *te = true;
+  te_start_kernel<T><<<1, 1, 0, b->stream>>>((TeInst<T> *)b->d_insts, first, v.parity, rows);
+  b->launches++;
+  b->psi_flips = 0;
+  int flips = 0;
+  return finish_run<T>(b, steps, views, &flips);
+}
+
 }  // namespace
+
+int fdtd_solo_run(fdtd_batch **batch, fdtd_ctx *ctx, bool check, int64_t steps, int64_t first,
+                  bool *te, long long *launches) {
+  if (!*batch) {
+    InstanceView v;
+    if (int r = fdtd_instance_view(ctx, &v)) return r;
+    fdtd_batch *b = new fdtd_batch();
+    b->solo = true;
+    b->ctxs.push_back(ctx);
+    b->precision = v.precision;
+    b->stream = v.stream;
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess)
+      cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev);
+    *batch = b;
+  }
+  fdtd_batch *b = *batch;
+  const long long before = b->launches;
+  const int r = b->precision == 64 ? solo_run<double>(b, check, steps, first, te)
+                                   : solo_run<float>(b, check, steps, first, te);
+  *launches += b->launches - before;
+  return r;
+}
 
 extern "C" {
 
@@ -1522,7 +1795,8 @@ int fdtd_batch_set_tile(fdtd_batch *b, int32_t width, int32_t height) {
     return 0;
   }
   for (int s = 0; s < NSHAPES; s++)
-    if (SHAPES[s].tw == width && SHAPES[s].th == height) {
+    if (SHAPES[s].tw == width && SHAPES[s].th == height &&
+        s != (b->precision == 64 ? BLOCK_TALL : BLOCK_LARGE)) {
       b->shape = s;
       return 0;
     }
@@ -1542,7 +1816,7 @@ void fdtd_batch_destroy(fdtd_batch *b) {
   for (cudaEvent_t ev : b->member_ev) cudaEventDestroy(ev);
   if (b->d_flags) cudaFreeAsync(b->d_flags, b->stream);
   if (b->stream) cudaStreamSynchronize(b->stream);
-  if (b->stream) cudaStreamDestroy(b->stream);
+  if (b->stream && !b->solo) cudaStreamDestroy(b->stream);
   delete b;
 }
 
@@ -1565,6 +1839,7 @@ struct fdtd_adjoint {
   int64_t first = 0;  // the forward run's first step index
   bool forward_done = false;
   long long ndesign = 0;
+  std::vector<long long> design;
   long long *d_design = nullptr;
   void *d_K = nullptr;          // segment x ndesign curls
   double *d_grad = nullptr;     // ndesign
@@ -1680,7 +1955,7 @@ int backward_impl(fdtd_adjoint *a, const double *grad_sums, double *grad_cb) {
                             b->stream));
   ATRY(a, cudaStreamSynchronize(b->stream));
   const int TW = 64, TH = 8;
-  const int tiles = ((v.n[0] + TW - 1) / TW) * ((v.n[1] + TH - 1) / TH);
+  const int tiles_x = (v.n[0] + TW - 1) / TW, tiles = tiles_x * ((v.n[1] + TH - 1) / TH);
   int per_sm = 1, dev = 0, sms = 148;
   ATRY(a, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, te_adjoint_kernel<T, 64, 8>,
                                                         THREADS, 0));
@@ -1694,6 +1969,7 @@ int backward_impl(fdtd_adjoint *a, const double *grad_sums, double *grad_cb) {
     if (int r = checkpoint(a, k, false)) return r;
     b->record = false;
     b->d_design = a->d_design;
+    b->design = &a->design;
     b->ndesign = a->ndesign;
     b->d_K = a->d_K;
     b->k_first = a->first + seg0;
@@ -1701,10 +1977,11 @@ int backward_impl(fdtd_adjoint *a, const double *grad_sums, double *grad_cb) {
     const int r = fdtd_batch_run(b, len, &at);
     b->record = true;
     b->d_design = nullptr;
+    b->design = nullptr;
     b->ndesign = 0;
     b->d_K = nullptr;
     if (r) return afail(a, r, "%s", fdtd_batch_last_error(b));
-    fdtd_instance_advance(a->ctx, -len);  // its probe record stays as the forward run left it
+    fdtd_instance_advance(a->ctx, -len, 0);  // its probe record stays as the forward run left it
     // that run's tables (the one simulation) hold what the adjoint reads
     const TeInst<T> *insts = (const TeInst<T> *)b->d_insts;
     if (v.nsums > 0 && v.nslots > 0) {
@@ -1718,7 +1995,7 @@ int backward_impl(fdtd_adjoint *a, const double *grad_sums, double *grad_cb) {
             insts, a->d_owner, a->d_start, a->d_order, a->nowners, a->d_phase, a->d_gsums, A, m);
       te_grad_kernel<T><<<(unsigned)((a->ndesign + 255) / 256), 256, 0, b->stream>>>(
           a->d_design, a->ndesign, (const T *)a->d_K + (long long)m * a->ndesign, A, a->d_grad);
-      te_adjoint_kernel<T, 64, 8><<<blocks, THREADS, 0, b->stream>>>(insts, A, tiles);
+      te_adjoint_kernel<T, 64, 8><<<blocks, THREADS, 0, b->stream>>>(insts, A, tiles_x, tiles);
       A.cur = 1 - A.cur;
     }
     ATRY(a, cudaGetLastError());
@@ -1778,6 +2055,7 @@ int fdtd_adjoint_create(fdtd_ctx *ctx, int64_t steps, int32_t segment, int64_t c
       return afail(a, FDTD_E_INVALID, "design value (%d, %d) is in a CPML", x, y);
   }
   a->ndesign = count;
+  a->design = design;
   const size_t E = v.precision == 64 ? 8 : 4;
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   a->ckpt_bytes = up(2 * v.N * E) + up(v.N * E) + up(v.psi_h_len * E) + up(v.psi_e_len * E);
@@ -1823,7 +2101,6 @@ int fdtd_adjoint_create(fdtd_ctx *ctx, int64_t steps, int32_t segment, int64_t c
   fdtd_ctx *one[1] = {ctx};
   if (int q = fdtd_batch_create(1, one, &a->batch))
     return afail(a, q, "%s", fdtd_batch_last_error(a->batch));
-  fdtd_batch_set_tile(a->batch, 64, 8);
   return 0;
 }
 

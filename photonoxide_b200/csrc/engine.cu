@@ -31,6 +31,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "photonoxide_batch.h"
 #include "photonoxide_fdtd.h"
 #include "common.cuh"
 #include "instance.h"
@@ -2129,56 +2130,94 @@ __device__ __forceinline__ double aux_difference(const double *f, long long o, d
 // (PlaneWaveRun::step_h then step_e, src/fdtd/sources.rs:1008-1040): before step m's H update the
 // slots of E its box's H couplings read, after it the slots of H its E couplings read, into the
 // step's values at nw + slot (stride values a step). The run's state stays on the device.
+// A step is a chain of three barriers and the differences' divisions on one SM, so what each wait
+// costs is what counts: with SHARED the state is in shared memory for the batch (48 bytes a
+// sample), a thread keeps its first AUX_KEPT slots' places in registers, and the sheet's waveform
+// is evaluated for all the batch's steps at once (a step of a 2400-sample run took 12 us with all
+// three from global memory, step by step).
+constexpr size_t AUX_SHARED = 224 * 1024;  // the most state kept in shared memory
+constexpr int AUX_KEPT = 4;
+constexpr int AUX_BATCH = 64;  // steps whose waveform is kept at a time
+template <bool SHARED>
 __global__ void __launch_bounds__(1024) aux_kernel(const AuxDev *runs, int nw, int stride,
                                                    long long first, const long long *base,
                                                    int batch, double dt, double *out_h,
                                                    double *out_e) {
+  extern __shared__ __align__(16) double aux_state[];
+  __shared__ double sheet_wave[AUX_BATCH];
   const AuxDev R = runs[blockIdx.x];
   if (base) first = *base;
-  const long long len = R.len, inner = len - 2 * R.pad;
+  const int len = (int)R.len, pad = (int)R.pad, inner = len - 2 * pad;
+  double *E = R.e, *H = R.h;
+  if (SHARED) {
+    E = aux_state;
+    H = aux_state + 3 * len;
+    for (int q = threadIdx.x; q < 3 * len; q += blockDim.x) {
+      E[q] = R.e[q];
+      H[q] = R.h[q];
+    }
+  }
+  int kept[AUX_KEPT];  // where the thread's slots are: E's place, or H's from 3 len on; -1 none
+#pragma unroll
+  for (int i = 0; i < AUX_KEPT; i++) {
+    const int q = threadIdx.x + i * blockDim.x;
+    kept[i] = q < R.nslots ? (R.slot_field[q] ? 3 * len : 0) + R.slot_comp[q] * len + (int)R.slot_i[q] : -1;
+  }
+  auto record = [&](int field, const double *f, double *out) {
+#pragma unroll
+    for (int i = 0; i < AUX_KEPT; i++) {
+      const int at = kept[i] - field * 3 * len;
+      if (kept[i] >= 0 && at >= 0 && at < 3 * len)
+        *reinterpret_cast<double2 *>(out + 2 * (threadIdx.x + i * blockDim.x)) = make_double2(f[at], 0.0);
+    }
+    for (int q = threadIdx.x + AUX_KEPT * blockDim.x; q < R.nslots; q += blockDim.x)
+      if (R.slot_field[q] == field)
+        *reinterpret_cast<double2 *>(out + 2 * q) =
+            make_double2(f[R.slot_comp[q] * len + R.slot_i[q]], 0.0);
+  };
   for (int m = 0; m < batch; m++) {
-    const double t = (double)(first + m) * dt, half = t + 0.5 * dt;
-    double *oh = out_h + 2LL * ((long long)m * stride + nw + R.slot0);
-    double *oe = out_e + 2LL * ((long long)m * stride + nw + R.slot0);
-    for (int q = threadIdx.x; q < R.nslots; q += blockDim.x)
-      if (R.slot_field[q] == 0) {
-        oh[2 * q] = R.e[R.slot_comp[q] * len + R.slot_i[q]];
-        oh[2 * q + 1] = 0.0;
+    if (m % AUX_BATCH == 0) {
+      const int q = threadIdx.x;
+      if (q < AUX_BATCH && m + q < batch && R.nsheet > 0) {  // the sheet's J at t + dt/2
+        double w, unused;
+        wave_eval(R.wave, (double)(first + m + q) * dt + 0.5 * dt, &w, &unused, 1);
+        sheet_wave[q] = w;
       }
-    for (long long q = threadIdx.x; q < 3 * inner; q += blockDim.x) {
-      const int c = (int)(q / inner);
-      const long long i = R.pad + q % inner;
+      __syncthreads();
+    }
+    record(0, E, out_h + 2LL * ((long long)m * stride + nw + R.slot0));
+    for (int q = threadIdx.x; q < 3 * inner; q += blockDim.x) {
+      const int c = q / inner, i = pad + q % inner;
       const int a = (c + 1) % 3, b = (c + 2) % 3;
-      const double curl = aux_difference(R.e + b * len, R.g[a], R.steps[a], i) -
-                          aux_difference(R.e + a * len, R.g[b], R.steps[b], i);
-      R.h[c * len + i] = R.da[i] * R.h[c * len + i] - R.db[i] * curl;
+      const double curl = aux_difference(E + b * len, R.g[a], R.steps[a], i) -
+                          aux_difference(E + a * len, R.g[b], R.steps[b], i);
+      H[c * len + i] = R.da[i] * H[c * len + i] - R.db[i] * curl;
     }
     __syncthreads();
-    for (int q = threadIdx.x; q < R.nslots; q += blockDim.x)
-      if (R.slot_field[q] == 1) {
-        oe[2 * q] = R.h[R.slot_comp[q] * len + R.slot_i[q]];
-        oe[2 * q + 1] = 0.0;
-      }
-    for (long long q = threadIdx.x; q < 3 * inner; q += blockDim.x) {
-      const int c = (int)(q / inner);
-      const long long i = R.pad + q % inner;
+    record(1, H, out_e + 2LL * ((long long)m * stride + nw + R.slot0));
+    for (int q = threadIdx.x; q < 3 * inner; q += blockDim.x) {
+      const int c = q / inner, i = pad + q % inner;
       const int a = (c + 1) % 3, b = (c + 2) % 3;
-      const double curl = aux_difference(R.h + b * len, R.g[a], R.steps[a], i) -
-                          aux_difference(R.h + a * len, R.g[b], R.steps[b], i);
-      R.e[c * len + i] = R.ca[i] * R.e[c * len + i] + R.cb[i] * curl;
+      const double curl = aux_difference(H + b * len, R.g[a], R.steps[a], i) -
+                          aux_difference(H + a * len, R.g[b], R.steps[b], i);
+      E[c * len + i] = R.ca[i] * E[c * len + i] + R.cb[i] * curl;
     }
     __syncthreads();
-    if (threadIdx.x == 0 && R.nsheet > 0) {  // the sheet's J at t + dt/2, one value at a time
-      double w, unused;
-      wave_eval(R.wave, half, &w, &unused, 1);
+    if (threadIdx.x == 0 && R.nsheet > 0) {  // one value at a time
+      const double w = sheet_wave[m % AUX_BATCH];
       for (int q = 0; q < R.nsheet; q++) {
         const long long i = R.sheet_i[q];
-        double &v = R.e[R.sheet_comp[q] * len + i];
+        double &v = E[R.sheet_comp[q] * len + i];
         v = v - R.cb[i] * R.sheet_j[q] * w;
       }
     }
     __syncthreads();
   }
+  if (SHARED)
+    for (int q = threadIdx.x; q < 3 * len; q += blockDim.x) {
+      R.e[q] = E[q];
+      R.h[q] = H[q];
+    }
 }
 
 // One coupling across a Bloch side (Bloch::wrap, src/fdtd/bloch.rs:97-152): value r of
@@ -2349,6 +2388,8 @@ __global__ void verify_division_kernel(float h, float r, double rd, int *bad) {
 // ------------------------------------------------------------------------------------------
 // The context: the device state of one simulation.
 
+constexpr long long SOLO_STEPS = 16;  // the shortest run that goes to the TE tiles (solo_ok)
+
 struct DeviceSlab {
   int field, comp, axis;
   long long from, count, psi, coef, size;
@@ -2411,6 +2452,13 @@ struct fdtd_ctx {
   std::vector<AuxDev> aux;
   std::vector<void *> aux_memory;
   AuxDev *d_aux = nullptr;
+  bool aux_te = true;      // no plane wave drives E_z, H_x or H_y
+  long long aux_len = 0;   // the longest run's samples
+  // a 2D TE run's own batch (solo_run): its tables, made on the first such run; te_known: the fields
+  // are TE and nothing but the engine has written them since that was looked up
+  fdtd_batch *solo = nullptr;
+  bool solo_off = false, te_known = false;
+  bool forced = false;  // a kernel was asked for by name
   int stride() const { return nwaves + naux + nbloch; }
   // probes and transforms
   int nprobes = 0;
@@ -2860,6 +2908,35 @@ int empty_sources(fdtd_ctx *c) {
   return 0;
 }
 
+// `batch` steps of the plane waves' auxiliary runs, their state in shared memory while it fits.
+void launch_aux(fdtd_ctx *c, int stride, long long first, const long long *base, int batch,
+                double *out_h, double *out_e) {
+  const size_t smem = (size_t)c->aux_len * 48;
+  if (smem <= AUX_SHARED)
+    aux_kernel<true><<<c->naux_runs, 1024, smem, c->stream>>>(c->d_aux, c->nwaves, stride, first,
+                                                              base, batch, c->dt, out_h, out_e);
+  else
+    aux_kernel<false><<<c->naux_runs, 1024, 0, c->stream>>>(c->d_aux, c->nwaves, stride, first,
+                                                            base, batch, c->dt, out_h, out_e);
+}
+
+// Whether `steps` steps may go to the TE tiles: a grid one cell thick and periodic there with
+// sources on E_x, E_y and H_z alone, none of the parts the tiles don't step, and enough steps to
+// pay for looking the fields up (about 25 us a run, against 10 us a step on the quad kernel).
+bool solo_ok(const fdtd_ctx *c, long long steps) {
+  if (c->solo_off || c->forced || c->profiling || c->capturing || steps < SOLO_STEPS) return false;
+  if (c->n[2] != 1 || !c->periodic[2] || c->media || c->nbloch > 0) return false;
+  if (c->naux_runs > 0 && !c->aux_te) return false;
+  for (const fdtd_injection &x : c->src_inj)
+    if ((x.field == 1) != (x.component == 2) && x.point != 2) return false;
+  if (c->budget) {
+    // E's psi again, and per monitored value its record, item and 32 steps
+    const size_t more = c->psi_e_len * c->elem + (size_t)c->nvalues * (64 + 32 * c->elem) + (1u << 20);
+    if (c->used + more > c->budget) return false;
+  }
+  return true;
+}
+
 template <typename T>
 int run_impl(fdtd_ctx *c, long long steps, long long first) {
   if (!c->coeffs_set || !c->fields_set)
@@ -2869,6 +2946,23 @@ int run_impl(fdtd_ctx *c, long long steps, long long first) {
   if (c->nbloch > 0)
     return fail(c, FDTD_E_STATE, "a context with Bloch couplings steps with fdtd_bloch_run");
   c->sums_fresh = true;
+  if (solo_ok(c, steps)) {
+    bool te = false;
+    const int r = fdtd_solo_run(&c->solo, c, !c->te_known, steps, first, &te, &c->launches);
+    if (te) {
+      c->te_known = true;
+      return r == 0 ? 0 : fail(c, r, "a run on the TE tiles: %s", fdtd_batch_last_error(c->solo));
+    }
+    if (r) {  // no room for its tables: nothing has run, and the general path serves
+      cudaGetLastError();
+      fdtd_batch_destroy(c->solo);
+      c->solo = nullptr;
+      c->solo_off = true;
+    }
+  }
+  if (c->te_known)  // the fields stay TE under TE sources only
+    for (const fdtd_injection &x : c->src_inj)
+      if ((x.field == 1) != (x.component == 2)) c->te_known = false;
   const int K = c->ring_k > 0 ? c->ring_k : 64;
   // the probes' record: grow to the run's steps
   if (c->nprobes > 0 && c->recorded + steps > c->record_cap) {
@@ -2892,9 +2986,7 @@ int run_impl(fdtd_ctx *c, long long steps, long long first) {
       c->launches++;
     }
     if (c->naux_runs > 0) {
-      aux_kernel<<<c->naux_runs, 1024, 0, c->stream>>>(c->d_aux, c->nwaves, c->stride(),
-                                                       first + at, base, batch, c->dt,
-                                                       c->waves_h, c->waves_e);
+      launch_aux(c, c->stride(), first + at, base, batch, c->waves_h, c->waves_e);
       c->launches++;
     }
     for (int m = 0; m < batch; m++) {
@@ -3312,6 +3404,7 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
         (long long)c->n[0] * c->n[1] < (1LL << 31);
     std::string kind = force ? force : (quad_ok ? "quad" : "row");
     if (kind == "quad" && !quad_ok) kind = "row";
+    c->forced = force != nullptr;
     c->quad = kind == "quad";
     c->row = kind == "row";
     c->staged = kind == "staged" && (c->n[0] % (16 / (int)c->elem) == 0);
@@ -3361,6 +3454,7 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
 void fdtd_destroy(fdtd_ctx *c) {
   if (!c) return;
   if (c->stream) cudaStreamSynchronize(c->stream);
+  fdtd_batch_destroy(c->solo);
   for (cudaEvent_t ev : c->events) cudaEventDestroy(ev);
   for (double *p : c->host_stage)
     if (p) cudaFreeHost(p);
@@ -3394,6 +3488,7 @@ int fdtd_upload_fields(fdtd_ctx *c, const double *e, const double *h, const doub
   if (!c) return FDTD_E_INVALID;
   c->generation++;
   c->parity = 0;
+  c->te_known = false;
   size_t E = c->elem;
   if (e) { if (int r = upload(c, c->e[0], e, 3 * c->N)) return r; }
   else CUDA_TRY(c, cudaMemsetAsync(c->e[0], 0, 3 * c->N * E, c->stream));
@@ -3635,6 +3730,8 @@ int fdtd_set_plane_waves(fdtd_ctx *c, int32_t count, const fdtd_plane_wave *w) {
   c->d_aux = nullptr;
   c->naux_runs = 0;
   c->naux = 0;
+  c->aux_te = true;
+  c->aux_len = 0;
   auto put = [&](const void *src, size_t bytes, void **dst) -> int {
     if (int r = alloc(c, dst, bytes)) return r;
     c->aux_memory.push_back(*dst);
@@ -3687,12 +3784,23 @@ int fdtd_set_plane_waves(fdtd_ctx *c, int32_t count, const fdtd_plane_wave *w) {
     if (int r = put(x.slot_i, (size_t)x.nslots * 8, &p)) return r;
     d.slot_i = (const long long *)p;
     slots += x.nslots;
+    c->aux_len = std::max<long long>(c->aux_len, x.len);
+    // whether the run has E_z, H_x or H_y: driven, there already, or turned up by a z component
+    for (int q = 0; q < x.nsheet; q++)
+      if (x.sheet_comp[q] == 2 && x.sheet_j[q] != 0.0) c->aux_te = false;
+    for (long long q = 0; q < x.len; q++)
+      if ((x.e0 && x.e0[2 * x.len + q] != 0.0) || (x.h0 && (x.h0[q] != 0.0 || x.h0[x.len + q] != 0.0)))
+        c->aux_te = false;
+    if (x.g[2] != 0) c->aux_te = false;
     c->aux.push_back(d);
   }
   if (count > 0) {
     if (int r = alloc(c, (void **)&c->d_aux, count * sizeof(AuxDev))) return r;
     CUDA_TRY(c, copy(c, c->d_aux, c->aux.data(), count * sizeof(AuxDev), cudaMemcpyHostToDevice));
   }
+  if (count > 0 && (size_t)c->aux_len * 48 <= AUX_SHARED)
+    CUDA_TRY(c, cudaFuncSetAttribute(aux_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)AUX_SHARED));
   c->naux_runs = count;
   c->naux = slots;
   return 0;
@@ -3979,6 +4087,7 @@ int fdtd_read_dft(fdtd_ctx *c, double *sums, int64_t count) {
 
 int fdtd_device_fields(fdtd_ctx *c, void **e, void **h) {
   if (!c) return FDTD_E_INVALID;
+  c->te_known = false;  // the caller may write through them
   if (e) *e = c->e[c->parity];
   if (h) *h = c->h[c->parity];
   return 0;
@@ -4076,6 +4185,7 @@ extern "C" int fdtd_upload_fields_static(fdtd_ctx *c, const double *e, const dou
     if (int r = static_stage_address(c, &stage)) return r;
   c->generation++;
   c->parity = 0;
+  c->te_known = false;
   const size_t E = c->elem;
   const double *src[2] = {e, h};
   void *dst[2] = {c->e[0], c->h[0]};
@@ -4154,9 +4264,17 @@ int fdtd_instance_view(fdtd_ctx *c, InstanceView *v) {
   v->probes = c->d_probes;
   v->media = c->media;
   v->plane_waves = c->naux_runs > 0;
+  v->naux = c->naux;
   v->stream = c->stream;
+  v->layout = c->layout;
   v->generation = c->generation;
   return 0;
+}
+
+int fdtd_instance_aux(fdtd_ctx *c, int stride, const long long *base, int count, double *out_h,
+                      double *out_e) {
+  launch_aux(c, stride, 0, base, count, out_h, out_e);
+  return 1;
 }
 
 int fdtd_instance_reserve(fdtd_ctx *c, long long steps, double **rows) {
@@ -4179,10 +4297,10 @@ int fdtd_instance_reserve(fdtd_ctx *c, long long steps, double **rows) {
   return 0;
 }
 
-void fdtd_instance_advance(fdtd_ctx *c, long long steps) {
+void fdtd_instance_advance(fdtd_ctx *c, long long steps, int flips) {
   if (!c) return;
   c->sums_fresh = true;
-  if (steps & 1) c->parity = 1 - c->parity;
+  if (flips & 1) c->parity = 1 - c->parity;
   if (c->nprobes > 0) c->recorded += steps;
 }
 

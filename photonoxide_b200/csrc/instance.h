@@ -39,17 +39,31 @@ struct InstanceView {
   const long long *probes;
   bool media;
   bool plane_waves;  // total-field/scattered-field boxes (stepped by the engine alone)
+  int naux;            // the values a step of its auxiliary runs records (te_block tiles only)
   cudaStream_t stream;
+  unsigned long long layout;      // moves on with the calls that change what a batch's tables hold
   unsigned long long generation;  // moves on with every change the engine's calls make
 };
 
 int fdtd_instance_view(fdtd_ctx *c, InstanceView *v);
 // The probe record's rows for `steps` more steps (grown as needed); null without probes.
 int fdtd_instance_reserve(fdtd_ctx *c, long long steps, double **rows);
-// After `steps` steps taken by the batch: the current copies and the record's length.
-void fdtd_instance_advance(fdtd_ctx *c, long long steps);
+// After `steps` steps taken by the batch, the current copy having changed `flips` times: the
+// current copies and the record's length.
+void fdtd_instance_advance(fdtd_ctx *c, long long steps, int flips);
 // The transforms' sums since the last read added into `parts` (doubles, interleaved, laid end to
 // end in the layout of fdtd_read_dft; lens: each part's), the device's then zero. Does nothing
 // where no step has been taken since the last read.
+// `count` steps of the context's plane waves' auxiliary runs from step *base (device memory), their
+// values into the tables of `stride` values a step after the emitters'; the kernels launched.
+int fdtd_instance_aux(fdtd_ctx *c, int stride, const long long *base, int count, double *out_h,
+                      double *out_e);
+// A 2D TE context's own steps on the batch's tiles of several steps a launch, enqueued on its stream
+// (batch.cu). *batch: made on the first call, the context's to destroy. check: whether the fields may
+// have come from elsewhere since the last such run: that H_x, H_y, E_z are zero is then looked up
+// (and waited for); *te false: they are not, and nothing has run. Adds its launches to *launches.
+struct fdtd_batch;
+int fdtd_solo_run(fdtd_batch **batch, fdtd_ctx *c, bool check, int64_t steps, int64_t first,
+                  bool *te, long long *launches);
 int fdtd_instance_add_dft(fdtd_ctx *c, int nparts, double *const *parts, const long long *lens);
 int fdtd_instance_fail(fdtd_ctx *c, int code, const char *what);
