@@ -891,6 +891,7 @@ __global__ void te_grad_kernel(const long long *design, long long n, const T *K,
 }  // namespace pxb
 
 #include "te_block.cuh"
+#include "te_adjoint_block.cuh"
 
 namespace pxb {
 
@@ -1377,6 +1378,7 @@ void launch_block(fdtd_batch *b, int m, int count, int launch) {
   A.k_first = b->k_first;
   A.ndesign = b->ndesign;
   A.record = b->record ? 1 : 0;
+  A.ahead = b->sms;
   kernel<<<b->ntiles, NW * 32, smem, b->stream>>>((const TeInst<T> *)b->d_insts, b->d_tile_inst, A, m,
                                                   count, launch);
 }
@@ -1849,6 +1851,15 @@ struct fdtd_adjoint {
   long long *d_owner = nullptr, *d_order = nullptr;
   int *d_start = nullptr;
   int nowners = 0;
+  // te_adjoint_block_kernel's tables by tile, and per step of a segment its amounts and E~ at the
+  // design (block: made; else the steps go one by one)
+  bool block = false;
+  int shape = 0, tiles = 0, tiles_x = 0;
+  long long norder = 0;
+  int *d_obucket = nullptr, *d_omid = nullptr, *d_dbucket = nullptr;
+  AdjOwner *d_owners = nullptr;
+  TeDesign *d_ditems = nullptr;
+  void *d_amount = nullptr, *d_kept = nullptr;
   // checkpoints: E_x, E_y, H_z, H's psi and E's psi at the start of each segment, and at the end
   void *d_ckpt = nullptr;
   size_t ckpt_bytes = 0;
@@ -1929,6 +1940,99 @@ int forward_impl(fdtd_adjoint *a, int64_t first) {
   return 0;
 }
 
+template <typename T, int HALO, int ROWS>
+void adjoint_block(cudaStream_t stream, const TeInst<T> *insts, const AdjState<T> &A,
+                   const AdjTables<T> &B, int tiles, int m, int count) {
+  constexpr int NW = BLOCK_WARPS<T>, R = ROWS / NW;
+  auto kernel = te_adjoint_block_kernel<T, NW, R, HALO>;
+  constexpr size_t smem = block_smem_values<T, NW, R>() * sizeof(T);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  kernel<<<tiles, NW * 32, smem, stream>>>(insts, A, B, m, count);
+}
+
+// The tables of te_adjoint_block_kernel, where the amounts of a segment's steps take no more than
+// ADJOINT_AMOUNTS bytes and the device has room; otherwise the steps go one by one.
+constexpr size_t ADJOINT_AMOUNTS = 256u << 20;
+int adjoint_tables(fdtd_adjoint *a, const InstanceView &v, const std::vector<long long> &owner,
+                   const std::vector<int> &start) {
+  const size_t E = a->precision == 64 ? 8 : 4;
+  a->norder = start.empty() ? 0 : start.back();
+  if ((size_t)a->segment * (size_t)a->norder * E > ADJOINT_AMOUNTS) return 0;
+  int dev = 0, sms = 148;
+  ATRY(a, cudaGetDevice(&dev));
+  ATRY(a, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  a->shape = block_shape({v}, sms);
+  const int TW = SHAPES[a->shape].tw, TH = SHAPES[a->shape].th, halo = SHAPES[a->shape].halo;
+  const int nx = v.n[0], ny = v.n[1];
+  a->tiles_x = (nx + TW - 1) / TW;
+  const int tiles_y = (ny + TH - 1) / TH;
+  a->tiles = a->tiles_x * tiles_y;
+  // the places of every region that hold a value, wrapped images included (build)
+  auto images = [&](int c, int n, int w, int len, int tiles, int periodic) {
+    std::vector<std::pair<int, int>> out;
+    for (int t = 0; t < tiles; t++) {
+      const int lo = t * w - halo;
+      if (!periodic) {
+        if (c >= lo && c < lo + len) out.push_back({t, c - lo});
+        continue;
+      }
+      int first = (c - lo) % n;
+      if (first < 0) first += n;
+      for (int q = first; q < len; q += n) out.push_back({t, q});
+    }
+    return out;
+  };
+  std::vector<std::vector<AdjOwner>> eo(a->tiles), ho(a->tiles);
+  for (size_t g = 0; g < owner.size(); g++) {
+    const bool hf = (owner[g] >> 62) != 0;
+    const long long place = owner[g] & ((1LL << 62) - 1), r = place % v.N;
+    const int comp = hf ? 2 : (int)(place / v.N);
+    for (auto oy : images((int)(r / nx), ny, TH, TH + 2 * halo, tiles_y, v.periodic[1]))
+      for (auto ox : images((int)(r % nx), nx, TW, BW, a->tiles_x, v.periodic[0]))
+        (hf ? ho : eo)[oy.first * a->tiles_x + ox.first].push_back(
+            AdjOwner{oy.second * BW + ox.second, comp, start[g], start[g + 1] - start[g]});
+  }
+  std::vector<std::vector<TeDesign>> dp(a->tiles);
+  for (long long d = 0; d < a->ndesign; d++) {
+    const long long r = a->design[d] % v.N;
+    const int x = (int)(r % nx), y = (int)(r / nx), tx = x / TW, ty = y / TH;
+    dp[ty * a->tiles_x + tx].push_back(
+        TeDesign{(y - ty * TH + halo) * BW + x - tx * TW + halo, (int)(a->design[d] / v.N), d});
+  }
+  std::vector<int> ob{0}, om, db{0};
+  std::vector<AdjOwner> owners;
+  std::vector<TeDesign> items;
+  for (int t = 0; t < a->tiles; t++) {
+    owners.insert(owners.end(), eo[t].begin(), eo[t].end());
+    om.push_back((int)owners.size());
+    owners.insert(owners.end(), ho[t].begin(), ho[t].end());
+    ob.push_back((int)owners.size());
+    items.insert(items.end(), dp[t].begin(), dp[t].end());
+    db.push_back((int)items.size());
+  }
+  bool ok = true;
+  auto put = [&](void **dst, const void *src, size_t bytes) {
+    *dst = nullptr;
+    if (!ok) return;
+    if (cudaMalloc(dst, std::max<size_t>(bytes, 16)) != cudaSuccess) {
+      cudaGetLastError();
+      ok = false;
+      return;
+    }
+    a->allocs.push_back(*dst);
+    if (src && bytes && cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) ok = false;
+  };
+  put((void **)&a->d_obucket, ob.data(), ob.size() * 4);
+  put((void **)&a->d_omid, om.data(), om.size() * 4);
+  put((void **)&a->d_dbucket, db.data(), db.size() * 4);
+  put((void **)&a->d_owners, owners.data(), owners.size() * sizeof(AdjOwner));
+  put((void **)&a->d_ditems, items.data(), items.size() * sizeof(TeDesign));
+  put(&a->d_amount, nullptr, (size_t)a->segment * a->norder * E);
+  put(&a->d_kept, nullptr, (size_t)a->segment * a->ndesign * E);
+  a->block = ok;
+  return 0;
+}
+
 template <typename T>
 int backward_impl(fdtd_adjoint *a, const double *grad_sums, double *grad_cb) {
   fdtd_batch *b = a->batch;
@@ -1989,7 +2093,32 @@ int backward_impl(fdtd_adjoint *a, const double *grad_sums, double *grad_cb) {
       te_segment_phase_kernel<T><<<(total + 127) / 128, 128, 0, b->stream>>>(insts, at, len,
                                                                             a->d_phase);
     }
-    for (int m = len - 1; m >= 0; m--) {
+    if (a->block) {
+      if (a->norder > 0)
+        te_amount_kernel<T><<<(unsigned)((a->norder * len + 255) / 256), 256, 0, b->stream>>>(
+            insts, a->d_order, a->norder, a->d_phase, a->d_gsums, len, (T *)a->d_amount);
+      AdjTables<T> B;
+      B.obucket = a->d_obucket;
+      B.dbucket = a->d_dbucket;
+      B.omid = a->d_omid;
+      B.owner = a->d_owners;
+      B.design = a->d_ditems;
+      B.amount = (const T *)a->d_amount;
+      B.norder = a->norder;
+      B.kept = (T *)a->d_kept;
+      B.ndesign = a->ndesign;
+      B.tiles_x = a->tiles_x;
+      const int halo = SHAPES[a->shape].halo;
+      for (int m = len - 1; m >= 0; m -= halo) {
+        const int count = std::min(halo, m + 1);
+        if (a->shape == BLOCK_SMALL) adjoint_block<T, 8, 32>(b->stream, insts, A, B, a->tiles, m, count);
+        else adjoint_block<T, 4, sizeof(T) == 4 ? 48 : 32>(b->stream, insts, A, B, a->tiles, m, count);
+        A.cur = 1 - A.cur;
+      }
+      te_grad_sum_kernel<T><<<(unsigned)((a->ndesign + 127) / 128), 128, 0, b->stream>>>(
+          a->ndesign, (const T *)a->d_kept, (const T *)a->d_K, len, a->d_grad);
+    }
+    for (int m = len - 1; m >= 0 && !a->block; m--) {
       if (v.nsums > 0 && a->nowners > 0)
         te_inject_kernel<T><<<(unsigned)((a->nowners + 255) / 256), 256, 0, b->stream>>>(
             insts, a->d_owner, a->d_start, a->d_order, a->nowners, a->d_phase, a->d_gsums, A, m);
@@ -2070,6 +2199,8 @@ int fdtd_adjoint_create(fdtd_ctx *ctx, int64_t steps, int32_t segment, int64_t c
   if (int q = amalloc(a, &a->d_adj, (size_t)2 * (3 * v.N + pe + ph) * E)) return q;
   ATRY(a, cudaMemcpy(a->d_design, design.data(), count * 8, cudaMemcpyHostToDevice));
   // the field values the transforms record, each with its transform values in value order
+  std::vector<long long> owner, order;
+  std::vector<int> start(1, 0);
   if (v.nvalues > 0 && v.nsums > 0) {
     std::vector<long long> where(v.nvalues);
     ATRY(a, cudaMemcpy(where.data(), v.where, v.nvalues * 8, cudaMemcpyDeviceToHost));
@@ -2081,8 +2212,6 @@ int fdtd_adjoint_create(fdtd_ctx *ctx, int64_t steps, int32_t segment, int64_t c
       if (hfield ? comp != 2 : comp == 2) continue;  // E_z, H_x, H_y: zero whatever eps
       by_place[where[q]].push_back(q);
     }
-    std::vector<long long> owner, order;
-    std::vector<int> start(1, 0);
     for (const auto &kv : by_place) {
       owner.push_back(kv.first);
       order.insert(order.end(), kv.second.begin(), kv.second.end());
@@ -2098,6 +2227,7 @@ int fdtd_adjoint_create(fdtd_ctx *ctx, int64_t steps, int32_t segment, int64_t c
       ATRY(a, cudaMemcpy(a->d_start, start.data(), start.size() * 4, cudaMemcpyHostToDevice));
     }
   }
+  if (int q = adjoint_tables(a, v, owner, start)) return q;
   fdtd_ctx *one[1] = {ctx};
   if (int q = fdtd_batch_create(1, one, &a->batch))
     return afail(a, q, "%s", fdtd_batch_last_error(a->batch));

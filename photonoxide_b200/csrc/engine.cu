@@ -3442,6 +3442,9 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
   c->zchunks = (c->n[2] + c->zchunk - 1) / c->zchunk;
   if (c->quad) {
     c->zchunks = quad_runs(c, chunks);
+    // short runs: no more CTAs than the device holds at once (the CPMLs' runs come on top)
+    if (c->n[2] / 4 < slots / tiles)
+      for (int q = chunks - 1; q > 1 && c->zchunks * tiles > slots; q--) c->zchunks = quad_runs(c, q);
     const std::vector<int> order = quad_order(c);
     if (int r = alloc(c, (void **)&c->order, order.size() * 4)) return r;
     CUDA_TRY(c, copy(c, c->order, order.data(), order.size() * 4, cudaMemcpyHostToDevice));

@@ -48,6 +48,7 @@ struct BlockArgs {
   T *K;
   long long k_first, ndesign;
   int record;  // 0: no values recorded
+  int ahead;   // the tile a CTA after this one's SM takes next, about: its rows are brought into L2
 };
 
 constexpr int BW = 128;  // places along x of a tile's region: four a lane
@@ -106,6 +107,24 @@ __device__ __forceinline__ void block_psi(T *psi, T *diff_u, const V4<T> &b, con
   }
   stv(psi, old.v);
   stv(diff_u, u);
+}
+
+// A warp's places in an x slab, shared out: the few lanes that hold some (`lanes`; `in` which of a
+// lane's four) times the warp's rows, an item a lane at a time, rather than row after row by those
+// lanes alone (a row's psi is a chain of some 300 cycles however few lanes take it). f(row, holder,
+// its `in`) for each item in the grid.
+template <int R, typename F>
+__device__ __forceinline__ void block_x_items(unsigned lanes, int in, int flags, int lane, F f) {
+  const int n = __popc(lanes), first = n ? __ffs(lanes) - 1 : 0;
+  const bool run = (lanes >> first) == (n < 32 ? (1u << n) - 1u : ~0u);  // one run of lanes
+#pragma unroll 1
+  for (int base = 0; base < n * R; base += 32) {
+    const int it = base + lane, r = it / n, k = it - r * n;
+    const bool valid = it < n * R;
+    const int holder = !valid ? lane : run ? first + k : (int)__fns(lanes, 0, k + 1);
+    const int its = __shfl_sync(0xffffffffu, in, holder);
+    if (valid && (flags >> (4 * r) & 1)) f(r, holder, its);
+  }
 }
 
 // g wrapped into 0 .. n-1 (from any number of periods away), or -1 beyond a wall.
@@ -265,12 +284,29 @@ __global__ void __launch_bounds__(NW * 32, 1)
   const int er0 = B.record ? B.erecs[tile] : 0, er1 = B.record ? B.erecs[tile + 1] : 0;
   const int d0 = B.dbucket ? B.dbucket[tile] : 0, d1 = B.dbucket ? B.dbucket[tile + 1] : 0;
   const bool lay_h = hg1 > hg0 || hr1 > hr0 || d1 > d0, lay_e = eg1 > eg0 || er1 > er0;
+  if (HALO == 4 && tile + B.ahead < (int)gridDim.x) {
+    // one CTA an SM loads, steps and stores in turn; the next one's rows, a 128-byte line a lane
+    // (2400 x 2400 places: 30.1 -> 27.0 us a step; eight steps a launch hide it anyway)
+    const TeInst<T> &Q = insts[tile_inst[tile + B.ahead]];
+    const int t = tile + B.ahead - Q.tile0;
+    const int x0 = max((t % Q.tiles_x) * OWNX - HALO, 0), x1 = min((t % Q.tiles_x) * OWNX - HALO + BW, Q.nx);
+    const int y0 = (t / Q.tiles_x) * OWNY - HALO + w * R, c = (Q.parity + launch) & 1;
+    constexpr int LINE = 128 / (int)sizeof(T), LINES = BW / LINE + 1;
+#pragma unroll 1
+    for (int q = lane; q < 5 * R * LINES; q += 32) {
+      const int a = q / (R * LINES), y = y0 + q / LINES % R, x = min(x0 + q % LINES * LINE, x1 - 1);
+      const T *f = a < 2 ? Q.e[c] + a * Q.N : a == 2 ? Q.h[c] + 2 * Q.N : Q.cb + (a - 3) * Q.N;
+      if (y >= 0 && y < Q.ny)
+        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(f + (long long)y * Q.nx + x));
+    }
+  }
   const T *ca = I.ca;
   const T sx = I.sx, sy = I.sy, inv_sx = I.inv_sx, inv_sy = I.inv_sy;
   const int fast_x = I.fast_x, fast_y = I.fast_y;
   stv(row_e + w * BW + 4 * lane, ex[0]);
   const bool any_held = __syncthreads_or(held);
-  // whether the warp has a slab's places
+  // whether the warp has a slab's places, and the lanes that have an x slab's
+  const unsigned lanes_h = __ballot_sync(0xffffffffu, inhx != 0), lanes_e = __ballot_sync(0xffffffffu, inex != 0);
   const bool slab_h = __any_sync(0xffffffffu, inhx != 0 || (flags & 0x2222)),
              slab_e = __any_sync(0xffffffffu, inex != 0 || (flags & 0x4444));
 
@@ -302,9 +338,6 @@ __global__ void __launch_bounds__(NW * 32, 1)
 #pragma unroll 1
       for (int r = 0; r < R; r++) {
         T *d = pub + slots + r * BW;
-        if (inhx && (flags >> (4 * r) & 1))
-          block_psi<T>(psi_hx + slots + r * BW, d, ldv(xco + 4 * lane), ldv(xco + BW + 4 * lane), sx,
-                       inv_sx, I.rd_x, fast_x, T(1), T(0), inhx);
         if (flags >> (4 * r) & 2) {
           const T b = yco[8 * (w * R + r)], a = yco[8 * (w * R + r) + 1];
           const V4<T> bb = {{b, b, b, b}}, aa = {{a, a, a, a}};
@@ -312,6 +345,13 @@ __global__ void __launch_bounds__(NW * 32, 1)
                        okx);
         }
       }
+      __syncwarp();
+      block_x_items<R>(lanes_h, inhx, flags, lane, [&](int r, int q, int in) {
+        const int at = (w * R + r) * BW + 4 * q;
+        block_psi<T>(psi_hx + at, pub + at, ldv(xco + 4 * q), ldv(xco + BW + 4 * q), sx, inv_sx, I.rd_x,
+                     fast_x, T(1), T(0), in);
+      });
+      __syncwarp();
 #pragma unroll
       for (int r = 0; r < R; r++) {
         if (inhx && (flags >> (4 * r) & 1)) {
@@ -436,10 +476,14 @@ __global__ void __launch_bounds__(NW * 32, 1)
           block_psi<T>(psi_ey + slots + r * BW, d + AREA, bb, aa, sy, inv_sy, I.rd_y, fast_y, T(1), T(-0.0),
                        okx);
         }
-        if (inex && (flags >> (4 * r) & 1))
-          block_psi<T>(psi_ex + slots + r * BW, d, ldv(xco + 2 * BW + 4 * lane),
-                       ldv(xco + 3 * BW + 4 * lane), sx, inv_sx, I.rd_x, fast_x, T(-1), T(-0.0), inex);
       }
+      __syncwarp();
+      block_x_items<R>(lanes_e, inex, flags, lane, [&](int r, int q, int in) {
+        const int at = (w * R + r) * BW + 4 * q;
+        block_psi<T>(psi_ex + at, pub + at, ldv(xco + 2 * BW + 4 * q), ldv(xco + 3 * BW + 4 * q), sx,
+                     inv_sx, I.rd_x, fast_x, T(-1), T(-0.0), in);
+      });
+      __syncwarp();
 #pragma unroll
       for (int r = 0; r < R; r++) {
         if (flags >> (4 * r) & 4) {
