@@ -116,6 +116,7 @@ struct SeriesDev {
   int slot0;         // its phases' slot for frequency 0
 };
 
+#ifdef __CUDACC__
 // A transform's value over a batch of steps: for N frequencies from the one whose phases start at
 // ph (2 doubles a frequency, `slots` frequencies a step), the sums at acc (a frequency's `volume`
 // complex sums apart) += sum over the steps of ring[m] ph[m], f64, in time order. The value's N
@@ -172,6 +173,7 @@ __device__ __forceinline__ void transform_value(const T *ring, long long row, in
   if (count & 1)
     transform_chunk<T, 1>(ring, row, batch, ph + 2 * f, slots, acc + 2 * f * volume, volume);
 }
+#endif
 
 // x / h with h a grid step, the quotient IEEE division gives. In f32, where `fast` (set only
 // after the engine has compared it with division for every finite float x, see
@@ -213,34 +215,51 @@ __host__ __device__ __forceinline__ double div_by_step(double x, double h, doubl
   return x / h;
 }
 
-// Four quotients x[j] / h at once, each div_by_step's: where all four take its common path (x
-// zero, or not tiny with a normal quotient) that path's three operations each and one test for
-// the four; otherwise div_by_step value by value. The same bits either way. (Zero differences
-// are the rule where the fields are still at rest, as in most of a CPML early in a run.)
-__host__ __device__ __forceinline__ void div4_by_step(const float x[4], float q[4], float h, float r,
-                                                      double rd, int fast) {
-  if (fast) {
-    bool common = true;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const float q0 = x[j] * r;
-      const float e = fmaf(-q0, h, x[j]);
-      const float qj = fmaf(e, r, q0);
-      const float aq = fabsf(qj);
-      const bool zero = x[j] == 0.0f;  // x r, its sign kept: q0
-      q[j] = zero ? q0 : qj;
-      common = common &&
-               (zero || (fabsf(x[j]) >= 0x1p-90f && aq >= 0x1p-126f && aq <= 3.40282347e38f));
-    }
-    if (common) return;
-  }
-#pragma unroll
-  for (int j = 0; j < 4; j++) q[j] = div_by_step(x[j], h, r, rd, fast);
+#ifdef __CUDACC__
+// x / h as the product with rd = 1/h in double, rounded once to float: the product is within 2^-52 of
+// the quotient, and a normal quotient of two 24-bit numbers lies further than that from every midpoint
+// of two floats, so it rounds as the division does; zeros keep their sign, what overflows does. Compared
+// with division for every finite x, subnormal quotients included, before it is used
+// (verify_division_kernel). Three instructions and no branch, where div_by_step's rare values take some
+// thirty each.
+__device__ __forceinline__ float div_product(float x, double rd) { return (float)((double)x * rd); }
+__device__ __forceinline__ float div_one(float x, float h, double rd, int fast) {
+  return fast ? div_product(x, rd) : x / h;
 }
-__host__ __device__ __forceinline__ void div4_by_step(const double x[4], double q[4], double h,
+__device__ __forceinline__ double div_one(double x, double h, double, int) { return x / h; }
+
+// Four quotients x[j] / h at once: where all four are zero or not tiny with a normal quotient (div_by_step's
+// common path) that path's three operations each and one test for the four; otherwise (a field that has
+// died away beside one that has not) by div_product. The same bits either way. (Zero differences are
+// the rule where the fields are still at rest, as in most of a CPML early in a run.)
+__device__ __forceinline__ void div4_by_step(const float x[4], float q[4], float h, float r, double rd,
+                                             int fast) {
+  if (!fast) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) q[j] = PXF_DIV_RARE(x[j], h);
+    return;
+  }
+  bool common = true;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const float q0 = x[j] * r;
+    const float e = fmaf(-q0, h, x[j]);
+    const float qj = fmaf(e, r, q0);
+    const float aq = fabsf(qj);
+    const bool zero = x[j] == 0.0f;  // x r, its sign kept: q0
+    q[j] = zero ? q0 : qj;
+    common = common &&
+             (zero || (fabsf(x[j]) >= 0x1p-90f && aq >= 0x1p-126f && aq <= 3.40282347e38f));
+  }
+  if (common) return;
+#pragma unroll
+  for (int j = 0; j < 4; j++) q[j] = div_product(x[j], rd);
+}
+__device__ __forceinline__ void div4_by_step(const double x[4], double q[4], double h,
                                                       double, double, int) {
 #pragma unroll
   for (int j = 0; j < 4; j++) q[j] = x[j] / h;
 }
+#endif
 
 }  // namespace pxf

@@ -1397,7 +1397,7 @@ __device__ __forceinline__ void xcoop(const StepArgs<T> &A, int k, int my, int x
       const T old = xp[(FIELD * 2 + (c - 1)) * 16 + (lane - (c - 1) * P)];  // staged
       const T *r = c == 1 ? r1 : r2;
       const T d = FIELD == 1 ? r[pos + 1] - r[pos] : r[pos] - r[pos - 1];
-      const T q = div_by_step(d, A.step[0], A.inv_step[0], A.inv_step64[0], A.fast_div[0]);
+      const T q = div_one(d, A.step[0], A.inv_step64[0], A.fast_div[0]);
       const T nw = b * old + a * q;
       u = (c == 1 ? T(-1) : T(1)) * nw;
       if (write && (pos >> 2) >= 1) (FIELD == 1 ? A.psi_h_out : A.psi_e)[at] = nw;
@@ -2371,8 +2371,8 @@ __global__ void add_into_kernel(const double *dev, double *host, long long n) {
 
 using namespace pxf;
 
-// For every finite float x: whether div_by_step's product form (reciprocal r) gives x / h's
-// bits. Sets *bad if any x differs. 2^32 values, a few milliseconds on a B200.
+// For every finite float x: whether div_by_step's product form (reciprocal r) and div_product's
+// give x / h's bits. Sets *bad if any x differs. 2^32 values, a few milliseconds on a B200.
 __global__ void verify_division_kernel(float h, float r, double rd, int *bad) {
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   int found = 0;
@@ -2380,7 +2380,9 @@ __global__ void verify_division_kernel(float h, float r, double rd, int *bad) {
        i < (1ULL << 32); i += stride) {
     const float x = __uint_as_float((unsigned)i);
     if (!isfinite(x)) continue;
-    if (__float_as_uint(div_by_step(x, h, r, rd, 1)) != __float_as_uint(x / h)) found = 1;
+    const unsigned want = __float_as_uint(x / h);
+    if (__float_as_uint(div_by_step(x, h, r, rd, 1)) != want || __float_as_uint(div_product(x, rd)) != want)
+      found = 1;
   }
   if (found) atomicOr(bad, 1);
 }
@@ -4310,10 +4312,10 @@ void fdtd_instance_advance(fdtd_ctx *c, long long steps, int flips) {
 namespace {
 constexpr long long HOST_CHUNK = 1LL << 18;  // doubles: 2 MiB
 
-// n doubles of src added into the parts laid end to end, from place `at` of them on. Large runs
-// over the host's threads: one core adds at a fraction of what the link delivers.
+// n doubles of src added into the parts laid end to end, from place `at` of them on; wide: over the
+// host's threads, where one core adds at a fraction of what the link delivers.
 void add_into_parts(const double *src, long long at, long long n, int nparts, double *const *parts,
-                    const long long *lens) {
+                    const long long *lens, bool wide) {
   long long base = 0;
   for (int p = 0; p < nparts && base < at + n; base += lens[p], p++) {
     const long long lo = std::max(at, base), hi = std::min(at + n, base + lens[p]);
@@ -4321,7 +4323,7 @@ void add_into_parts(const double *src, long long at, long long n, int nparts, do
     double *to = parts[p] + (lo - base);
     const double *from = src + (lo - at);
     const long long m = hi - lo;
-#pragma omp parallel for schedule(static) if (m > (1 << 16))
+#pragma omp parallel for schedule(static) if (wide && m > (1 << 15))
     for (long long q = 0; q < m; q++) to[q] += from[q];
   }
 }
@@ -4362,7 +4364,8 @@ int fdtd_instance_add_dft(fdtd_ctx *c, int nparts, double *const *parts, const l
   for (long long at = 0; at < n; at += HOST_CHUNK) {
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (at + HOST_CHUNK < n) CUDA_TRY(c, get(at + HOST_CHUNK));
-    add_into_parts(buf[(at / HOST_CHUNK) & 1], at, std::min(HOST_CHUNK, n - at), nparts, parts, lens);
+    add_into_parts(buf[(at / HOST_CHUNK) & 1], at, std::min(HOST_CHUNK, n - at), nparts, parts, lens,
+                   n > (1 << 19));
   }
   CUDA_TRY(c, cudaMemsetAsync(c->sums, 0, c->nsums * 16, c->stream));
   c->sums_fresh = false;

@@ -60,35 +60,6 @@ __host__ __device__ constexpr size_t block_smem_values() {
   return (size_t)6 * NW * R * BW + (2 * NW + 1) * BW + 6 * BW + 8 * NW * R;
 }
 
-// x[j] / h for four values, div_by_step's bits (div4_by_step, the rare values in a loop: this kernel's
-// step has to stay short, see te_block_kernel).
-__device__ __forceinline__ void block_div4(const float x[4], float q[4], float h, float r, double rd,
-                                           int fast) {
-  bool common = fast != 0;
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    const float q0 = x[j] * r;
-    const float qj = fmaf(fmaf(-q0, h, x[j]), r, q0), aq = fabsf(qj);
-    const bool zero = x[j] == 0.0f;
-    q[j] = zero ? q0 : qj;
-    common = common && (zero || (fabsf(x[j]) >= 0x1p-90f && aq >= 0x1p-126f && aq <= 3.40282347e38f));
-  }
-  if (common) return;
-#pragma unroll 1
-  for (int j = 0; j < 4; j++) {
-    const float v = div_by_step(j == 0 ? x[0] : j == 1 ? x[1] : j == 2 ? x[2] : x[3], h, r, rd, fast);
-    if (j == 0) q[0] = v;
-    else if (j == 1) q[1] = v;
-    else if (j == 2) q[2] = v;
-    else q[3] = v;
-  }
-}
-__device__ __forceinline__ void block_div4(const double x[4], double q[4], double h, double, double,
-                                           int) {
-#pragma unroll
-  for (int j = 0; j < 4; j++) q[j] = x[j] / h;
-}
-
 // A slab's psi at four places: psi <- b psi + a (d/h) where `in`; u, in the differences' place, is
 // what the field's update takes: sign psi, or elsewhere a zero that leaves the field as it is (H
 // subtracts dt u: +0; E adds cb u: -0).
@@ -98,7 +69,7 @@ __device__ __forceinline__ void block_psi(T *psi, T *diff_u, const V4<T> &b, con
   V4<T> old = ldv(psi);
   const V4<T> diff = ldv(diff_u);
   T d[4], u[4];
-  block_div4(diff.v, d, h, inv, rd, fast);
+  div4_by_step(diff.v, d, h, inv, rd, fast);
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     const T nw = b.v[j] * old.v[j] + a.v[j] * d[j];
