@@ -29,7 +29,7 @@ int fdtd_batch_create(int32_t count, fdtd_ctx *const *ctxs, fdtd_batch **out);
 const char *fdtd_batch_last_error(const fdtd_batch *batch);
 /* `steps` steps of every grid; grid i's first step has index first_steps[i] (its step count so
  * far, as fdtd_run's first_step), all 0 when first_steps is NULL. A batch whose tile shape is not set
- * takes tiles of several steps a launch (below). Returns
+ * takes one by its size, of several steps a launch but for few cells in f64. Returns
  * once the steps are queued: each context's stream waits for them, so its later calls (reads,
  * runs, fdtd_synchronize) come after. */
 int fdtd_batch_run(fdtd_batch *batch, int64_t steps, const int64_t *first_steps);

@@ -903,7 +903,7 @@ struct Shape {
 // taller tile's values have no registers, 120 x 40 in f32)
 const Shape SHAPES[] = {{32, 8, 0}, {32, 16, 0}, {64, 4, 0}, {64, 8, 0}, {128, 2, 0}, {128, 4, 0},
                         {teq::OWN, teq::RW, 0}, {112, 16, 8}, {120, 24, 4}, {120, 40, 4}};
-constexpr int QUAD_SHAPE = 6, BLOCK_SMALL = 7, BLOCK_LARGE = 8, BLOCK_TALL = 9;
+constexpr int ONE_STEP = 3, QUAD_SHAPE = 6, BLOCK_SMALL = 7, BLOCK_LARGE = 8, BLOCK_TALL = 9;
 constexpr int NSHAPES = sizeof(SHAPES) / sizeof(SHAPES[0]);
 // te_block_kernel's warps: f32, 16 of 2 rows (eight steps a launch) or 3 (four: fewer halo places);
 // f64, 8 of 4 rows.
@@ -1534,16 +1534,25 @@ int finish_run(fdtd_batch *b, int64_t steps, const std::vector<InstanceView> &vi
   return 0;
 }
 
-// The tile shape of a batch whose caller fixed none: te_block_kernel's, eight steps a launch while
-// its tiles fill the SMs a few times over, four steps beyond (us a step, eight against four, f32: one
-// 537 x 541 grid 6.6 and 9.8; 1.29 M cells in six 17.8 and 18.3; 2.6 M in twelve 33.7 and 32.4; 19.2 M
-// in 64 217 and 195; one step a launch 12.2, 29.9, 54.3 and 373).
-int block_shape(const std::vector<InstanceView> &views, int sms) {
-  long long tiles = 0;
-  for (const InstanceView &v : views)
-    tiles += (long long)((v.n[0] + SHAPES[BLOCK_SMALL].tw - 1) / SHAPES[BLOCK_SMALL].tw) *
-             ((v.n[1] + SHAPES[BLOCK_SMALL].th - 1) / SHAPES[BLOCK_SMALL].th);
-  return tiles <= 6LL * sms ? BLOCK_SMALL : views[0].precision == 64 ? BLOCK_LARGE : BLOCK_TALL;
+// The tile shape of a batch whose caller fixed none. f32: te_block_kernel's, eight steps a launch while
+// its tiles fill the SMs a few times over, four steps beyond (us a step, eight against four: one
+// 537 x 541 grid 6.6 and 9.2; 1.29 M cells in six 17.7 and 17.9; 2.6 M in twelve 33.1 and 32.0; 19.2 M
+// in 64 212 and 186; one step a launch 12.2, 30.6, 54.2 and 374). f64, where a tile has half the warps:
+// four steps a launch from about 1.3 M cells on (40.2 us against one step's 40.2; 3.4 M cells 85.5 and
+// 98.9, 10.4 M 209 and 266), one step below (0.16 M cells 16.9 and 11.4).
+int block_shape(const std::vector<InstanceView> &views, int sms, bool one_step) {
+  auto tiles = [&](int shape) {
+    long long n = 0;
+    for (const InstanceView &v : views)
+      n += (long long)((v.n[0] + SHAPES[shape].tw - 1) / SHAPES[shape].tw) *
+           ((v.n[1] + SHAPES[shape].th - 1) / SHAPES[shape].th);
+    return n;
+  };
+  if (views[0].precision == 64) {
+    if (one_step && tiles(BLOCK_LARGE) <= 4LL * sms) return ONE_STEP;
+    return tiles(BLOCK_SMALL) <= sms ? BLOCK_SMALL : BLOCK_LARGE;
+  }
+  return tiles(BLOCK_SMALL) <= 6LL * sms ? BLOCK_SMALL : BLOCK_TALL;
 }
 
 // A run whose members are all as the last run left them: its tables and graph serve again, the
@@ -1640,7 +1649,7 @@ int run_impl(fdtd_batch *b, int64_t steps, const int64_t *first_steps) {
         return bfail(b, FDTD_E_INVALID,
                      "simulation %d has H_x, H_y or E_z values: the batch steps TE fields only", i);
   }
-  if (b->shape < 0) b->shape = block_shape(views, b->sms);
+  if (b->shape < 0) b->shape = block_shape(views, b->sms, true);
   if (int r = build<T>(b, views, first, parity, rows, b->shape)) return r;
   if (SHAPES[b->shape].halo > 0) launch_shape<T>(b, 0, 0, 0);
   else b->blocks = occupancy<T>(b) * b->sms;
@@ -1704,7 +1713,7 @@ int solo_run(fdtd_batch *b, bool check, int64_t steps, int64_t first, bool *te) 
   if (!b->reusable || b->solo_layout != v.layout) {
     b->reusable = false;
     b->aux = v.naux > 0;
-    b->shape = block_shape(views, b->sms);
+    b->shape = block_shape(views, b->sms, false);
     if (int r = build<T>(b, views, {first}, {v.parity}, {rows}, b->shape)) return r;
     launch_shape<T>(b, 0, 0, 0);
     b->solo_layout = v.layout;
@@ -1961,7 +1970,7 @@ int adjoint_tables(fdtd_adjoint *a, const InstanceView &v, const std::vector<lon
   int dev = 0, sms = 148;
   ATRY(a, cudaGetDevice(&dev));
   ATRY(a, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  a->shape = block_shape({v}, sms);
+  a->shape = block_shape({v}, sms, false);
   const int TW = SHAPES[a->shape].tw, TH = SHAPES[a->shape].th, halo = SHAPES[a->shape].halo;
   const int nx = v.n[0], ny = v.n[1];
   a->tiles_x = (nx + TW - 1) / TW;
