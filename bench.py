@@ -530,7 +530,7 @@ def _te_instances(count, seed=0, precision=32):
 
 def workload_batch(args):
     """Configuration 4, forward: 64 uneven 2D TE instances (sides log-uniform 256-1024 cells) with
-    100x100 design regions, 6000 steps, batched (one persistent launch per step for all, CUDA-
+    100x100 design regions, 6000 steps, batched (several steps of all of them a launch, CUDA-
     graph chunks, tile shape by size) against the same instances run one at a time: through the
     3D engine (``one_at_a_time``) and as batches of one on the same TE kernel and tile shape
     (``one_at_a_time_te_kernel``, which isolates the batching's own gain)."""
@@ -644,7 +644,7 @@ def workload_serving(args):
     for sp, s in zip(specs, sims):
         if sp.two_d:
             def one():
-                Batch([s], tile=(124, 7) if s.grid.nx % 4 == 0 else (32, 16)).run(sp.steps)
+                Batch([s]).run(sp.steps)
                 s.transforms()
         else:
             def one():

@@ -204,7 +204,9 @@ int fdtd_set_media(fdtd_ctx *ctx, int32_t ngroups, const fdtd_media_group *group
  * sources' and transforms' times), as Resident::step (resident.rs:430-539). Returns when the
  * device is done. */
 int fdtd_run(fdtd_ctx *ctx, int64_t steps, int64_t first_step);
-/* The same, enqueued on the context's stream without waiting (for timing and overlap). */
+/* The same, enqueued on the context's stream without waiting (for timing and overlap). A 2D run of TE
+ * sources whose fields have come from elsewhere since its last run (uploaded, or handed out by
+ * fdtd_device_fields) first waits for the context's earlier work, to see whether they are TE. */
 int fdtd_run_async(fdtd_ctx *ctx, int64_t steps, int64_t first_step);
 int fdtd_synchronize(fdtd_ctx *ctx);
 
