@@ -46,6 +46,9 @@ constexpr int G = 32;  // steps per chunk (even: a chunk leaves the copies' pari
 template <typename T>
 struct TeInst {
   int nx, ny, px, py;  // sizes, periodic flags
+  // the low CPMLs' places along x and y: a place below is the low slab's, any other the high one's (a
+  // CPML may reach past the grid's middle, so the middle tells nothing)
+  int low_x, low_y;
   int pitch;           // values from a row of a y slab's psi to the next
   long long N;
   T dt, sx, sy;        // the step's dt and the grid steps along x and y, as the kernel rounds them
@@ -153,14 +156,14 @@ __global__ void __launch_bounds__(THREADS) te_step_kernel(
         const bool own = lx >= 1 && ly >= 1;
         // the CPML: H_z along x (+), then along y (-)
         if (!I.px) {
-          const int side = mx < nx / 2 ? 0 : 1;
+          const int side = mx < I.low_x ? 0 : 1;
           const SlabEntry &s = I.hx[side];
           if (in_slab(s, mx))
             hz = slab_h(I, s, mx, s.psi + (long long)my * s.pw + (mx - s.pf), pin, pout, own, dxEy,
                         0, T(1), hz);
         }
         if (!I.py) {
-          const int side = my < ny / 2 ? 0 : 1;
+          const int side = my < I.low_y ? 0 : 1;
           const SlabEntry &s = I.hy[side];
           if (in_slab(s, my))
             hz = slab_h(I, s, my, s.psi + (long long)(my - s.from) * I.pitch + mx, pin, pout, own, dyEx,
@@ -214,14 +217,14 @@ __global__ void __launch_bounds__(THREADS) te_step_kernel(
         T ney = cay * ein[N + r] + cby * curl1;
         // the CPML: E_x along y (+), E_y along x (-)
         if (!I.py) {
-          const int side = y < ny / 2 ? 0 : 1;
+          const int side = y < I.low_y ? 0 : 1;
           const SlabEntry &s = I.ey[side];
           if (in_slab(s, y))
             nex = slab_e(I, s, y, s.psi + (long long)(y - s.from) * I.pitch + x, I.psi_e, dyHz, 1,
                          T(1), cbx, nex);
         }
         if (!I.px) {
-          const int side = x < nx / 2 ? 0 : 1;
+          const int side = x < I.low_x ? 0 : 1;
           const SlabEntry &s = I.ex[side];
           if (in_slab(s, x))
             ney = slab_e(I, s, x, s.psi + (long long)y * s.pw + (x - s.pf), I.psi_e, dxHz, 0,
@@ -378,14 +381,14 @@ __global__ void __launch_bounds__(THREADS, 4) te_quad_kernel(
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           if (!ok[j]) continue;
-          const SlabEntry &s = I.hx[mx[j] < nx / 2 ? 0 : 1];
+          const SlabEntry &s = I.hx[mx[j] < I.low_x ? 0 : 1];
           if (in_slab(s, mx[j]))
             hz[j] = slab_h(I, s, mx[j], s.psi + (long long)my * s.pw + (mx[j] - s.pf), pin, pout,
                            own, dxEy[j], 0, T(1), hz[j]);
         }
       }
       if (!I.py) {
-        const SlabEntry &s = I.hy[my < ny / 2 ? 0 : 1];
+        const SlabEntry &s = I.hy[my < I.low_y ? 0 : 1];
         if (in_slab(s, my))
 #pragma unroll
           for (int j = 0; j < 4; j++)
@@ -447,7 +450,7 @@ __global__ void __launch_bounds__(THREADS, 4) te_quad_kernel(
       }
       // the CPML: E_x along y (+), E_y along x (-)
       if (!I.py) {
-        const SlabEntry &s = I.ey[my < ny / 2 ? 0 : 1];
+        const SlabEntry &s = I.ey[my < I.low_y ? 0 : 1];
         if (in_slab(s, my))
 #pragma unroll
           for (int j = 0; j < 4; j++)
@@ -459,7 +462,7 @@ __global__ void __launch_bounds__(THREADS, 4) te_quad_kernel(
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           if (!ok[j]) continue;
-          const SlabEntry &s = I.ex[mx[j] < nx / 2 ? 0 : 1];
+          const SlabEntry &s = I.ex[mx[j] < I.low_x ? 0 : 1];
           if (in_slab(s, mx[j]))
             ney[j] = slab_e(I, s, mx[j], s.psi + (long long)my * s.pw + (mx[j] - s.pf), I.psi_e,
                             dxHz[j], 0, T(-1), cby.v[j], ney[j]);
@@ -741,14 +744,14 @@ __global__ void __launch_bounds__(THREADS) te_adjoint_kernel(const TeInst<T> *in
         }
         // the E slabs: psi' = b psi + (a/h) (difference of H_z)
         if (!I.py) {
-          const SlabEntry &s0 = I.ey[my < ny / 2 ? 0 : 1];
+          const SlabEntry &s0 = I.ey[my < I.low_y ? 0 : 1];
           if (in_slab(s0, my)) {
             const T tot = psi_ex_total(mx, my, r, s0);
             acc = acc + coef_a(I, s0, my) / I.sy * tot;
             if (own) peo[s0.psi + (long long)(my - s0.from) * I.pitch + mx] = coef_b(I, s0, my) * tot;
           }
           if (myp >= 0) {
-            const SlabEntry &s1 = I.ey[myp < ny / 2 ? 0 : 1];
+            const SlabEntry &s1 = I.ey[myp < I.low_y ? 0 : 1];
             if (in_slab(s1, myp)) {
               const long long rp = (long long)myp * nx + mx;
               acc = acc - coef_a(I, s1, myp) / I.sy * psi_ex_total(mx, myp, rp, s1);
@@ -756,14 +759,14 @@ __global__ void __launch_bounds__(THREADS) te_adjoint_kernel(const TeInst<T> *in
           }
         }
         if (!I.px) {
-          const SlabEntry &s0 = I.ex[mx < nx / 2 ? 0 : 1];
+          const SlabEntry &s0 = I.ex[mx < I.low_x ? 0 : 1];
           if (in_slab(s0, mx)) {
             const T tot = psi_ey_total(mx, my, r, s0);
             acc = acc + coef_a(I, s0, mx) / I.sx * tot;
             if (own) peo[s0.psi + (long long)my * s0.pw + (mx - s0.pf)] = coef_b(I, s0, mx) * tot;
           }
           if (mxp >= 0) {
-            const SlabEntry &s1 = I.ex[mxp < nx / 2 ? 0 : 1];
+            const SlabEntry &s1 = I.ex[mxp < I.low_x ? 0 : 1];
             if (in_slab(s1, mxp)) {
               const long long rp = (long long)my * nx + mxp;
               acc = acc - coef_a(I, s1, mxp) / I.sx * psi_ey_total(mxp, my, rp, s1);
@@ -799,26 +802,26 @@ __global__ void __launch_bounds__(THREADS) te_adjoint_kernel(const TeInst<T> *in
       if (ym >= 0) ax = ax + I.dt * I.fh[nx + ym] * hy;
       if (xm >= 0) ay = ay - I.dt * I.fh[xm] * hx;
       if (!I.py) {
-        const SlabEntry &s0 = I.hy[y < ny / 2 ? 0 : 1];
+        const SlabEntry &s0 = I.hy[y < I.low_y ? 0 : 1];
         if (in_slab(s0, y)) {
           const T tot = psi_hy_total(x, y, hc, s0);
           ax = ax - coef_a(I, s0, y) / I.sy * tot;
           pho[s0.psi + (long long)(y - s0.from) * I.pitch + x] = coef_b(I, s0, y) * tot;
         }
         if (ym >= 0) {
-          const SlabEntry &s1 = I.hy[ym < ny / 2 ? 0 : 1];
+          const SlabEntry &s1 = I.hy[ym < I.low_y ? 0 : 1];
           if (in_slab(s1, ym)) ax = ax + coef_a(I, s1, ym) / I.sy * psi_hy_total(x, ym, hy, s1);
         }
       }
       if (!I.px) {
-        const SlabEntry &s0 = I.hx[x < nx / 2 ? 0 : 1];
+        const SlabEntry &s0 = I.hx[x < I.low_x ? 0 : 1];
         if (in_slab(s0, x)) {
           const T tot = psi_hx_total(x, y, hc, s0);
           ay = ay - coef_a(I, s0, x) / I.sx * tot;
           pho[s0.psi + (long long)y * s0.pw + (x - s0.pf)] = coef_b(I, s0, x) * tot;
         }
         if (xm >= 0) {
-          const SlabEntry &s1 = I.hx[xm < nx / 2 ? 0 : 1];
+          const SlabEntry &s1 = I.hx[xm < I.low_x ? 0 : 1];
           if (in_slab(s1, xm)) ay = ay + coef_a(I, s1, xm) / I.sx * psi_hx_total(xm, y, hx, s1);
         }
       }
@@ -1072,6 +1075,8 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
     I.pitch = v.pitch;
     I.px = v.periodic[0];
     I.py = v.periodic[1];
+    I.low_x = v.low[0];
+    I.low_y = v.low[1];
     I.N = v.N;
     I.dt = (T)v.dt;
     I.dt64 = v.dt;
