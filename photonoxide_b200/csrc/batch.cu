@@ -1247,6 +1247,10 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
       void *second = nullptr;
       BTRY(b, cudaMallocAsync(&second, std::max<size_t>(v.psi_e_len, 1) * E, b->stream));
       b->allocs.push_back(second);
+      // what the tiles don't step there (E_z's psi, the rows' padding) is the engine's, so that either
+      // copy may be handed back whole
+      if (v.psi_e_len > 0)
+        BTRY(b, cudaMemcpyAsync(second, v.psi_e, v.psi_e_len * E, cudaMemcpyDeviceToDevice, b->stream));
       b->psi2[i] = second;
       I.psi_e2 = (T *)second;
       std::vector<std::vector<TeRec>> hp(ntile), ep(ntile);
