@@ -1599,6 +1599,26 @@ int run_again(fdtd_batch *b, int64_t steps, const int64_t *first_steps, bool *ra
   return 0;
 }
 
+// The other copy's H_x, H_y and E_z, which the steps leave alone, as the current copy's are: the fields at
+// zero, H's psi the current one's. (Either copy may end as the current one, and the other's psi is whatever
+// the steps before an upload left there.)
+template <typename T>
+int settle_tm(fdtd_batch *b, const InstanceView &v) {
+  const size_t E = sizeof(T);
+  const int other = 1 - v.parity;
+  BTRY(b, cudaMemsetAsync((char *)v.h[other], 0, 2 * v.N * E, b->stream));
+  BTRY(b, cudaMemsetAsync((char *)v.e[other] + 2 * v.N * E, 0, v.N * E, b->stream));
+  for (int axis = 0; axis < 2; axis++)  // H_y's slabs along x, H_x's along y
+    for (int side = 0; side < 2; side++) {
+      const SlabEntry &s = v.table[1][1 - axis][axis][side];
+      const size_t len = axis == 0 ? (size_t)s.pw * v.n[1] : (size_t)s.count * v.pitch;
+      if (s.count > 0)
+        BTRY(b, cudaMemcpyAsync((T *)v.psi_h[other] + s.psi, (const T *)v.psi_h[v.parity] + s.psi, len * E,
+                                cudaMemcpyDeviceToDevice, b->stream));
+    }
+  return 0;
+}
+
 template <typename T>
 int run_impl(fdtd_batch *b, int64_t steps, const int64_t *first_steps) {
   bool ran = false;
@@ -1643,10 +1663,7 @@ int run_impl(fdtd_batch *b, int64_t steps, const int64_t *first_steps) {
     BTRY(b, cudaStreamWaitEvent(b->stream, b->member_ev[i], 0));
     te_tm_check_kernel<T><<<(unsigned)((v.N + 255) / 256), 256, 0, b->stream>>>(
         (const T *)v.e[v.parity], (const T *)v.h[v.parity], v.N, b->d_flags + i);
-    // the other copy's TM components stay zero too
-    const size_t E = sizeof(T);
-    BTRY(b, cudaMemsetAsync((char *)v.h[1 - v.parity], 0, 2 * v.N * E, b->stream));
-    BTRY(b, cudaMemsetAsync((char *)v.e[1 - v.parity] + 2 * v.N * E, 0, v.N * E, b->stream));
+    if (int r = settle_tm<T>(b, v)) return r;
   }
   {
     std::vector<int> bad(n, 0);
@@ -1687,7 +1704,7 @@ int solo_run(fdtd_batch *b, bool check, int64_t steps, int64_t first, bool *te) 
   const size_t E = sizeof(T);
   *te = false;
   if (check) {
-    // H_x, H_y and E_z, and their psi, all zero; then the other copies' fields are too
+    // H_x, H_y and E_z, and their psi, all zero; then the other copies are made so
     ZeroRanges R;
     R.count = 0;
     auto add = [&](const void *at, long long len) {
@@ -1714,8 +1731,7 @@ int solo_run(fdtd_batch *b, bool check, int64_t steps, int64_t first, bool *te) 
     BTRY(b, cudaMemcpyAsync(&bad, b->d_flags, 4, cudaMemcpyDeviceToHost, b->stream));
     BTRY(b, cudaStreamSynchronize(b->stream));
     if (bad) return 0;
-    BTRY(b, cudaMemsetAsync(v.h[1 - v.parity], 0, 2 * v.N * E, b->stream));
-    BTRY(b, cudaMemsetAsync((char *)v.e[1 - v.parity] + 2 * v.N * E, 0, v.N * E, b->stream));
+    if (int r = settle_tm<T>(b, v)) return r;
   }
   double *rows = nullptr;
   if (int r = fdtd_instance_reserve(b->ctxs[0], steps, &rows)) return r;

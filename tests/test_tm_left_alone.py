@@ -94,3 +94,25 @@ def test_psi_of_e_whatever_the_memory_held(tile, precision, steps):
         assert np.array_equal(x, y)
     for q in (a.e(2), a.h(0), a.h(1)):
         assert not q.any()
+
+
+@pytest.mark.parametrize("tile,precision,steps", ROUTES)
+def test_psi_of_h_of_an_earlier_tm_run(tile, precision, steps):
+    a, o = grid(precision), grid(precision)
+    r = np.arange(a.grid.cells())
+    for c in range(3):
+        a.set_field(Field.E, c, noise(r + c))
+        a.set_field(Field.H, c, noise(r + 90 + c))
+    a.run(7)
+    for s in (a, o):
+        te_fields(s)  # the upload starts psi anew
+    take(a, tile, steps)
+    silent_ez(o)
+    o.run(steps)
+    silent_ez(a)
+    for s in (a, o):
+        s.run(6)
+    for x, y in zip(all_fields(a), all_fields(o)):
+        assert np.array_equal(x, y)
+    for q in (a.e(2), a.h(0), a.h(1)):
+        assert not q.any()
