@@ -3115,6 +3115,7 @@ int bloch_impl(fdtd_ctx *a, fdtd_ctx *b, const std::vector<WrapDev> &hw,
     return fail(a, FDTD_E_INVALID, "the two parts of a complex run differ");
   CUDA_TRY(a, cudaStreamSynchronize(b->stream));
   a->sums_fresh = b->sums_fresh = true;
+  a->te_known = b->te_known = false;  // the steps below take sources and couplings of any component
   const cudaStream_t st = a->stream;
   const int K = a->ring_k > 0 ? a->ring_k : 64;
   if (int r = grow_record(a, steps)) return r;

@@ -7,7 +7,8 @@ import numpy as np
 import pytest
 
 from photonoxide_b200.batch import Batch
-from photonoxide_b200.fdtd import Simulation
+from photonoxide_b200.engine import Engine
+from photonoxide_b200.fdtd import Simulation, library
 from photonoxide_b200.types import (INF, Axis, Boundaries, Boxes, Cpml, Field, Grid3d, Periodic, Pml,
                                     Source, Waveform)
 from scenarios import noise
@@ -116,3 +117,39 @@ def test_psi_of_h_of_an_earlier_tm_run(tile, precision, steps):
         assert np.array_equal(x, y)
     for q in (a.e(2), a.h(0), a.h(1)):
         assert not q.any()
+
+
+class Waveform_(C.Structure):
+    _fields_ = [("kind", C.c_int32), ("p", C.c_double * 5)]
+
+
+class Injection(C.Structure):
+    _fields_ = [("field", C.c_int32), ("component", C.c_int32), ("r", C.c_int64), ("a_re", C.c_double),
+                ("a_im", C.c_double), ("emitter", C.c_int32), ("point", C.c_int32)]
+
+
+def test_a_te_run_after_tm_steps_through_the_complex_entry(monkeypatch):
+    """One context: TE steps, steps with an E_z source through fdtd_bloch_run, TE sources again. The
+    fields are no longer TE, and every component goes on."""
+    x = library()
+    out = []
+    for kernel in (None, "quad"):
+        if kernel:
+            monkeypatch.setenv("PHOTONOXIDE_FDTD_KERNEL", kernel)
+        re, im = grid(32), grid(32)
+        for s in (re, im):
+            te_fields(s)
+            s.run(20)
+        a, b = Engine(re.engine()), Engine(im.engine())
+        wave = Waveform_(2, (C.c_double * 5)(1.0, 1.0, 0.0, 0.0, 0.0))
+        ez = Injection(0, 2, 20 * 130 + 60, 1.0, 0.0, 0, 1)
+        assert x.fdtd_set_sources(C.c_void_p(a.ctx), 1, C.byref(wave), C.c_int64(1), C.byref(ez)) == 0
+        assert x.fdtd_bloch_run(C.c_void_p(a.ctx), C.c_void_p(b.ctx), 0, None, C.c_int64(20), C.c_int64(20)) == 0
+        assert x.fdtd_set_sources(C.c_void_p(a.ctx), 0, None, C.c_int64(0), None) == 0
+        a.run(24, 40)
+        n = 3 * re.grid.cells()
+        e, h = np.empty(n), np.empty(n)
+        a.download_fields(e, h)
+        out.append((e, h))
+        assert e[2 * n // 3:].any()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
