@@ -1727,6 +1727,7 @@ int solo_run(fdtd_batch *b, bool check, int64_t steps, int64_t first, bool *te) 
     int bad = 0;
     BTRY(b, cudaMemsetAsync(b->d_flags, 0, 4, b->stream));
     te_zero_kernel<T><<<dim3(64, R.count), 256, 0, b->stream>>>(R, b->d_flags);
+    b->launches++;
     BTRY(b, cudaGetLastError());
     BTRY(b, cudaMemcpyAsync(&bad, b->d_flags, 4, cudaMemcpyDeviceToHost, b->stream));
     BTRY(b, cudaStreamSynchronize(b->stream));

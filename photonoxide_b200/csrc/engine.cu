@@ -2456,10 +2456,12 @@ struct fdtd_ctx {
   AuxDev *d_aux = nullptr;
   bool aux_te = true;      // no plane wave drives E_z, H_x or H_y
   long long aux_len = 0;   // the longest run's samples
-  // a 2D TE run's own batch (solo_run): its tables, made on the first such run; te_known: the fields
-  // are TE and nothing but the engine has written them since that was looked up
+  // a 2D TE run's own batch (solo_run): its tables, made on the first such run; te: what the
+  // last look at the fields found (1 TE, -1 not; 0: not looked at, or written by others than the engine's
+  // steps of TE sources since)
   fdtd_batch *solo = nullptr;
-  bool solo_off = false, te_known = false;
+  bool solo_off = false;
+  int te = 0;
   bool forced = false;  // a kernel was asked for by name
   int stride() const { return nwaves + naux + nbloch; }
   // probes and transforms
@@ -2926,7 +2928,7 @@ void launch_aux(fdtd_ctx *c, int stride, long long first, const long long *base,
 // sources on E_x, E_y and H_z alone, none of the parts the tiles don't step, and enough steps to
 // pay for looking the fields up (about 25 us a run, against 10 us a step on the quad kernel).
 bool solo_ok(const fdtd_ctx *c, long long steps) {
-  if (c->solo_off || c->forced || c->profiling || c->capturing || steps < SOLO_STEPS) return false;
+  if (c->solo_off || c->forced || c->profiling || c->capturing || steps < SOLO_STEPS || c->te < 0) return false;
   if (c->n[2] != 1 || !c->periodic[2] || c->media || c->nbloch > 0) return false;
   if (c->naux_runs > 0 && !c->aux_te) return false;
   for (const fdtd_injection &x : c->src_inj)
@@ -2950,9 +2952,9 @@ int run_impl(fdtd_ctx *c, long long steps, long long first) {
   c->sums_fresh = true;
   if (solo_ok(c, steps)) {
     bool te = false;
-    const int r = fdtd_solo_run(&c->solo, c, !c->te_known, steps, first, &te, &c->launches);
+    const int r = fdtd_solo_run(&c->solo, c, c->te == 0, steps, first, &te, &c->launches);
     if (te) {
-      c->te_known = true;
+      c->te = 1;
       return r == 0 ? 0 : fail(c, r, "a run on the TE tiles: %s", fdtd_batch_last_error(c->solo));
     }
     if (r) {  // no room for its tables: nothing has run, and the general path serves
@@ -2960,11 +2962,13 @@ int run_impl(fdtd_ctx *c, long long steps, long long first) {
       fdtd_batch_destroy(c->solo);
       c->solo = nullptr;
       c->solo_off = true;
+    } else {
+      c->te = -1;  // looked at once, not on each run
     }
   }
-  if (c->te_known)  // the fields stay TE under TE sources only
+  if (c->te > 0)  // the fields stay TE under TE sources only
     for (const fdtd_injection &x : c->src_inj)
-      if ((x.field == 1) != (x.component == 2)) c->te_known = false;
+      if ((x.field == 1) != (x.component == 2)) c->te = 0;
   const int K = c->ring_k > 0 ? c->ring_k : 64;
   // the probes' record: grow to the run's steps
   if (c->nprobes > 0 && c->recorded + steps > c->record_cap) {
@@ -3115,7 +3119,7 @@ int bloch_impl(fdtd_ctx *a, fdtd_ctx *b, const std::vector<WrapDev> &hw,
     return fail(a, FDTD_E_INVALID, "the two parts of a complex run differ");
   CUDA_TRY(a, cudaStreamSynchronize(b->stream));
   a->sums_fresh = b->sums_fresh = true;
-  a->te_known = b->te_known = false;  // the steps below take sources and couplings of any component
+  a->te = b->te = 0;  // the steps below take sources and couplings of any component
   const cudaStream_t st = a->stream;
   const int K = a->ring_k > 0 ? a->ring_k : 64;
   if (int r = grow_record(a, steps)) return r;
@@ -3494,7 +3498,7 @@ int fdtd_upload_fields(fdtd_ctx *c, const double *e, const double *h, const doub
   if (!c) return FDTD_E_INVALID;
   c->generation++;
   c->parity = 0;
-  c->te_known = false;
+  c->te = 0;
   size_t E = c->elem;
   if (e) { if (int r = upload(c, c->e[0], e, 3 * c->N)) return r; }
   else CUDA_TRY(c, cudaMemsetAsync(c->e[0], 0, 3 * c->N * E, c->stream));
@@ -4093,7 +4097,7 @@ int fdtd_read_dft(fdtd_ctx *c, double *sums, int64_t count) {
 
 int fdtd_device_fields(fdtd_ctx *c, void **e, void **h) {
   if (!c) return FDTD_E_INVALID;
-  c->te_known = false;  // the caller may write through them
+  c->te = 0;  // the caller may write through them
   if (e) *e = c->e[c->parity];
   if (h) *h = c->h[c->parity];
   return 0;
@@ -4191,7 +4195,7 @@ extern "C" int fdtd_upload_fields_static(fdtd_ctx *c, const double *e, const dou
     if (int r = static_stage_address(c, &stage)) return r;
   c->generation++;
   c->parity = 0;
-  c->te_known = false;
+  c->te = 0;
   const size_t E = c->elem;
   const double *src[2] = {e, h};
   void *dst[2] = {c->e[0], c->h[0]};

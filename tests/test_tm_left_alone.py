@@ -153,3 +153,23 @@ def test_a_te_run_after_tm_steps_through_the_complex_entry(monkeypatch):
         out.append((e, h))
         assert e[2 * n // 3:].any()
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+def test_fields_that_are_not_te_are_looked_at_once(monkeypatch):
+    """A run of fields on E_z without sources: the first run's look at the fields is not repeated (a
+    kernel, and a wait that fdtd_run_async would make its caller pay on every run)."""
+    counts = []
+    for kernel in (None, "quad"):
+        if kernel:
+            monkeypatch.setenv("PHOTONOXIDE_FDTD_KERNEL", kernel)
+        s = grid(32)
+        r = np.arange(s.grid.cells())
+        s.set_field(Field.E, 2, noise(r))
+        s.run(40)
+        e = Engine(s.engine())
+        first = e.launches()
+        e.run(40, 40)
+        counts.append((first, e.launches(), s.e(2)))
+    (a1, a2, a), (o1, o2, o) = counts
+    assert a1 == o1 + 1 and a2 == o2
+    assert np.array_equal(a, o)
