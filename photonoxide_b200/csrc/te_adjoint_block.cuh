@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
   const int tile = blockIdx.x;
   const TeInst<T> &I = insts[0];
   const int X0 = (tile % B.tiles_x) * OWNX - HALO, Y0 = (tile / B.tiles_x) * OWNY - HALO;
-  const int nx = I.nx, ny = I.ny;
+  const int nx = I.nx, ny = I.ny, low_x = I.low_x, low_y = I.low_y;
   const long long N = I.N;
   const T dt = I.dt;
   const T *eb = A.e[A.cur], *hb = A.h[A.cur], *pei = A.pe[A.cur], *phi = A.ph[A.cur];
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
     if (m < 0) continue;
     okx |= 1 << j;
     if (!I.px) {
-      const int side = m < I.low_x ? 0 : 1;
+      const int side = m < low_x ? 0 : 1;
       if (in_slab(I.hx[side], m)) inhx |= 1 << j;
       if (in_slab(I.ex[side], m)) inex |= 1 << j;
     }
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
     if (my < 0) return 0;
     int f = 1;
     if (!I.py) {
-      const int side = my < I.low_y ? 0 : 1;
+      const int side = my < low_y ? 0 : 1;
       if (in_slab(I.hy[side], my)) f |= 2;
       if (in_slab(I.ey[side], my)) f |= 4;
     }
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int m = xb + j;  // (no slab along a periodic x)
-        const SlabEntry &s = I.hx[m < I.low_x ? 0 : 1], &t = I.ex[m < I.low_x ? 0 : 1];
+        const SlabEntry &s = I.hx[m < low_x ? 0 : 1], &t = I.ex[m < low_x ? 0 : 1];
         q[j] = inhx >> j & 1 ? phi[s.psi + (long long)my * s.pw + (m - s.pf)] : T(0);
         o[j] = inex >> j & 1 ? pei[t.psi + (long long)my * t.pw + (m - t.pf)] : T(0);
       }
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
       stv(psi_ex + slots + r * BW, o);
     }
     if (f & 6) {
-      const int side = my < I.low_y ? 0 : 1;
+      const int side = my < low_y ? 0 : 1;
       const SlabEntry &s = I.hy[side], &t = I.ey[side];
       if (f & 2) {
         get(phi + s.psi + (long long)(my - s.from) * I.pitch, 0, q);
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
     const int m = wrap_any(X0 + q, nx, I.px);
     T c[4] = {T(0), T(0), T(0), T(0)};
     if (m >= 0 && !I.px) {
-      const SlabEntry &s = I.hx[m < I.low_x ? 0 : 1], &t = I.ex[m < I.low_x ? 0 : 1];
+      const SlabEntry &s = I.hx[m < low_x ? 0 : 1], &t = I.ex[m < low_x ? 0 : 1];
       if (in_slab(s, m)) c[0] = coef_b(I, s, m), c[1] = coef_a(I, s, m) / I.sx;
       if (in_slab(t, m)) c[2] = coef_b(I, t, m), c[3] = coef_a(I, t, m) / I.sx;
     }
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
     const int m = wrap_any(Y0 + q, ny, I.py);
     T c[4] = {T(0), T(0), T(0), T(0)};
     if (m >= 0 && !I.py) {
-      const SlabEntry &s = I.hy[m < I.low_y ? 0 : 1], &t = I.ey[m < I.low_y ? 0 : 1];
+      const SlabEntry &s = I.hy[m < low_y ? 0 : 1], &t = I.ey[m < low_y ? 0 : 1];
       if (in_slab(s, m)) c[0] = coef_b(I, s, m), c[1] = coef_a(I, s, m) / I.sy;
       if (in_slab(t, m)) c[2] = coef_b(I, t, m), c[3] = coef_a(I, t, m) / I.sy;
     }
@@ -453,13 +453,13 @@ __global__ void __launch_bounds__(NW * 32, 1)
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int m = xb + j;
-        const SlabEntry &a = I.hx[m < I.low_x ? 0 : 1], &b = I.ex[m < I.low_x ? 0 : 1];
+        const SlabEntry &a = I.hx[m < low_x ? 0 : 1], &b = I.ex[m < low_x ? 0 : 1];
         if (inhx >> j & 1) pho[a.psi + (long long)y * a.pw + (m - a.pf)] = q.v[j];
         if (inex >> j & 1) peo[b.psi + (long long)y * b.pw + (m - b.pf)] = o.v[j];
       }
     }
     if (flags >> (4 * r) & 6) {
-      const int side = y < I.low_y ? 0 : 1;
+      const int side = y < low_y ? 0 : 1;
       const SlabEntry &a = I.hy[side], &b = I.ey[side];
       const V4<T> q = ldv(psi_hy + slots + r * BW), o = ldv(psi_ey + slots + r * BW);
 #pragma unroll

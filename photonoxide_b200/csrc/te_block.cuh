@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
   const TeInst<T> &I = insts[tile_inst[tile]];
   const int lt = tile - I.tile0;
   const int X0 = (lt % I.tiles_x) * OWNX - HALO, Y0 = (lt / I.tiles_x) * OWNY - HALO;
-  const int nx = I.nx, ny = I.ny;
+  const int nx = I.nx, ny = I.ny, low_x = I.low_x, low_y = I.low_y;
   const long long N = I.N;
   const int cur = (I.parity + launch) & 1, pcur = (I.psi_parity + launch) & 1;
   const T dt = I.dt;
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
     if (m < 0) continue;
     okx |= 1 << j;
     if (!I.px) {
-      const int side = m < I.low_x ? 0 : 1;
+      const int side = m < low_x ? 0 : 1;
       if (in_slab(I.hx[side], m)) inhx |= 1 << j;
       if (in_slab(I.ex[side], m)) inex |= 1 << j;
     }
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int m = xb + j;  // (no slab along a periodic x)
-        const SlabEntry &s = I.hx[m < I.low_x ? 0 : 1], &t = I.ex[m < I.low_x ? 0 : 1];
+        const SlabEntry &s = I.hx[m < low_x ? 0 : 1], &t = I.ex[m < low_x ? 0 : 1];
         q[j] = inhx >> j & 1 ? pin[s.psi + (long long)my * s.pw + (m - s.pf)] : T(0);
         o[j] = inex >> j & 1 ? pein[t.psi + (long long)my * t.pw + (m - t.pf)] : T(0);
       }
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
       keep(psi_ex, o, inex);
     }
     if (!I.py) {
-      const int side = my < I.low_y ? 0 : 1;
+      const int side = my < low_y ? 0 : 1;
       const SlabEntry &s = I.hy[side], &t = I.ey[side];
       T q[4];
       if (in_slab(s, my)) {
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
     const int m = wrap_any(X0 + q, nx, I.px);
     T c[4] = {T(0), T(0), T(0), T(0)};
     if (m >= 0 && !I.px) {
-      const SlabEntry &s = I.hx[m < I.low_x ? 0 : 1], &t = I.ex[m < I.low_x ? 0 : 1];
+      const SlabEntry &s = I.hx[m < low_x ? 0 : 1], &t = I.ex[m < low_x ? 0 : 1];
       if (in_slab(s, m)) c[0] = I.coefs[s.coef + m - s.from], c[1] = I.coefs[s.coef + s.count + m - s.from];
       if (in_slab(t, m)) c[2] = I.coefs[t.coef + m - t.from], c[3] = I.coefs[t.coef + t.count + m - t.from];
     }
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
     const int m = wrap_any(Y0 + q, ny, I.py);
     T c[4] = {T(0), T(0), T(0), T(0)};
     if (m >= 0 && !I.py) {
-      const SlabEntry &s = I.hy[m < I.low_y ? 0 : 1], &t = I.ey[m < I.low_y ? 0 : 1];
+      const SlabEntry &s = I.hy[m < low_y ? 0 : 1], &t = I.ey[m < low_y ? 0 : 1];
       if (in_slab(s, m)) c[0] = I.coefs[s.coef + m - s.from], c[1] = I.coefs[s.coef + s.count + m - s.from];
       if (in_slab(t, m)) c[2] = I.coefs[t.coef + m - t.from], c[3] = I.coefs[t.coef + t.count + m - t.from];
     }
@@ -543,13 +543,13 @@ __global__ void __launch_bounds__(NW * 32, 1)
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int m = xb + j;
-        const SlabEntry &a = I.hx[m < I.low_x ? 0 : 1], &b = I.ex[m < I.low_x ? 0 : 1];
+        const SlabEntry &a = I.hx[m < low_x ? 0 : 1], &b = I.ex[m < low_x ? 0 : 1];
         if (inhx >> j & 1) pout[a.psi + (long long)y * a.pw + (m - a.pf)] = q.v[j];
         if (inex >> j & 1) peout[b.psi + (long long)y * b.pw + (m - b.pf)] = o.v[j];
       }
     }
     if (flags >> (4 * r) & 6) {
-      const int side = y < I.low_y ? 0 : 1;
+      const int side = y < low_y ? 0 : 1;
       const SlabEntry &a = I.hy[side], &b = I.ey[side];
       const V4<T> q = ldv(psi_hy + slots + r * BW), o = ldv(psi_ey + slots + r * BW);
 #pragma unroll
