@@ -35,6 +35,7 @@
 #include "photonoxide_fdtd.h"
 #include "common.cuh"
 #include "instance.h"
+#include "readout.h"
 #include "portable.h"
 
 namespace pxf {
@@ -2510,6 +2511,7 @@ struct fdtd_ctx {
   // read and kept (fdtd_instance_add_dft); sums_fresh: steps have been taken since the last read
   double *host_stage[2] = {nullptr, nullptr};
   bool sums_fresh = true;
+  long long sums_taken = 0;  // doubles of the sums read and not cleared (pxr::read_add)
   // step-kernel timing: pairs of events around each launch while profiling
   bool profiling = false;
   std::vector<cudaEvent_t> events;
@@ -3918,6 +3920,7 @@ int fdtd_set_dft(fdtd_ctx *c, int32_t nseries, const fdtd_series *series, int32_
   c->nseries = nseries;
   c->nslots = (int)omega.size();
   c->nsums = sums;
+  c->sums_taken = 0;
   c->freq_chunks = 1;
   for (const SeriesDev &x : sd) c->freq_chunks = std::max(c->freq_chunks, (x.nf + DFT_F - 1) / DFT_F);
   if (values == 0) return 0;
@@ -4315,8 +4318,6 @@ void fdtd_instance_advance(fdtd_ctx *c, long long steps, int flips) {
 }
 
 namespace {
-constexpr long long HOST_CHUNK = 1LL << 18;  // doubles: 2 MiB
-
 // n doubles of src added into the parts laid end to end, from place `at` of them on; wide: over the
 // host's threads, where one core adds at a fraction of what the link delivers.
 void add_into_parts(const double *src, long long at, long long n, int nparts, double *const *parts,
@@ -4338,6 +4339,7 @@ void add_into_parts(const double *src, long long at, long long n, int nparts, do
 // whole-plane transform (400 x 200, six components, 21 frequencies: 161 MB) had gone through three
 // pageable arrays made for each read, twice a call.
 int fdtd_instance_add_dft(fdtd_ctx *c, int nparts, double *const *parts, const long long *lens) {
+  using pxr::CHUNK;
   if (!c) return FDTD_E_INVALID;
   const long long n = 2 * c->nsums;
   long long room = 0;
@@ -4346,10 +4348,10 @@ int fdtd_instance_add_dft(fdtd_ctx *c, int nparts, double *const *parts, const l
   if (n == 0 || !c->sums_fresh) return 0;
   std::vector<double> plain;  // short reads, and where page-locked memory is refused
   double *buf[2] = {nullptr, nullptr};
-  if (n > HOST_CHUNK / 8) {
+  if (n > CHUNK / 8) {
     for (int b = 0; b < 2; b++)
       if (!c->host_stage[b] &&
-          cudaHostAlloc((void **)&c->host_stage[b], HOST_CHUNK * 8, cudaHostAllocDefault) != cudaSuccess) {
+          cudaHostAlloc((void **)&c->host_stage[b], CHUNK * 8, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
         c->host_stage[b] = nullptr;
       }
@@ -4357,22 +4359,26 @@ int fdtd_instance_add_dft(fdtd_ctx *c, int nparts, double *const *parts, const l
     buf[1] = c->host_stage[1];
   }
   if (!buf[0] || !buf[1]) {
-    plain.resize(2 * std::min(n, HOST_CHUNK));
+    plain.resize(2 * std::min(n, CHUNK));
     buf[0] = plain.data();
     buf[1] = plain.data() + plain.size() / 2;
   }
-  auto get = [&](long long at) {
-    const long long m = std::min(HOST_CHUNK, n - at);
-    return cudaMemcpyAsync(buf[(at / HOST_CHUNK) & 1], c->sums + at, m * 8, cudaMemcpyDeviceToHost, c->stream);
+  auto fetch = [&](long long at, long long m, double *to) -> int {
+    CUDA_TRY(c, cudaMemcpyAsync(to, c->sums + at, m * 8, cudaMemcpyDeviceToHost, c->stream));
+    return 0;
   };
-  CUDA_TRY(c, get(0));
-  for (long long at = 0; at < n; at += HOST_CHUNK) {
+  auto wait = [&]() -> int {
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-    if (at + HOST_CHUNK < n) CUDA_TRY(c, get(at + HOST_CHUNK));
-    add_into_parts(buf[(at / HOST_CHUNK) & 1], at, std::min(HOST_CHUNK, n - at), nparts, parts, lens,
-                   n > (1 << 19));
-  }
-  CUDA_TRY(c, cudaMemsetAsync(c->sums, 0, c->nsums * 16, c->stream));
+    return 0;
+  };
+  auto add = [&](long long at, long long m, const double *from) {
+    add_into_parts(from, at, m, nparts, parts, lens, n > (1 << 19));
+  };
+  auto clear = [&](long long m) -> int {
+    CUDA_TRY(c, cudaMemsetAsync(c->sums, 0, m * 8, c->stream));
+    return 0;
+  };
+  if (int r = pxr::read_add(n, &c->sums_taken, buf, fetch, wait, add, clear)) return r;
   c->sums_fresh = false;
   return 0;
 }
