@@ -421,8 +421,8 @@ struct pxs_sim {
     return 0;
   }
 
-  // Adds the device's transform sums into the host's.
-  int pull_sums() {
+  // Adds the device's transform sums into the host's (wide: see fdtd_instance_add_dft).
+  int pull_sums(bool wide = true) {
     if (!ctx || !configured || series.empty()) return 0;
     std::vector<double *> parts;
     std::vector<long long> lens;
@@ -430,7 +430,7 @@ struct pxs_sim {
       parts.push_back(s.sums.data());
       lens.push_back((long long)s.sums.size());
     }
-    if (int r = fdtd_instance_add_dft(ctx, (int)parts.size(), parts.data(), lens.data()))
+    if (int r = fdtd_instance_add_dft(ctx, (int)parts.size(), parts.data(), lens.data(), wide))
       return fail(r, "%s", fdtd_last_error(ctx));
     return 0;
   }
@@ -716,7 +716,8 @@ struct pxs_sim {
     } else {
       fields_dropped = true;  // the host's copies are stale: reading them or running refuses
     }
-    if (int r = pull_sums()) return r;
+    // the serving loop reads jobs back in threads that end with the reads, several at once: one thread each
+    if (int r = pull_sums(false)) return r;
     if (int r = pull_plane_waves()) return r;
     aux_on_device = 0;
     fdtd_destroy(ctx);

@@ -51,9 +51,6 @@ int fdtd_instance_reserve(fdtd_ctx *c, long long steps, double **rows);
 // After `steps` steps taken by the batch, the current copy having changed `flips` times: the
 // current copies and the record's length.
 void fdtd_instance_advance(fdtd_ctx *c, long long steps, int flips);
-// The transforms' sums since the last read added into `parts` (doubles, interleaved, laid end to
-// end in the layout of fdtd_read_dft; lens: each part's), the device's then zero. Does nothing
-// where no step has been taken since the last read.
 // `count` steps of the context's plane waves' auxiliary runs from step *base (device memory), their
 // values into the tables of `stride` values a step after the emitters'; the kernels launched.
 int fdtd_instance_aux(fdtd_ctx *c, int stride, const long long *base, int count, double *out_h,
@@ -65,5 +62,9 @@ int fdtd_instance_aux(fdtd_ctx *c, int stride, const long long *base, int count,
 struct fdtd_batch;
 int fdtd_solo_run(fdtd_batch **batch, fdtd_ctx *c, bool check, int64_t steps, int64_t first,
                   bool *te, long long *launches);
-int fdtd_instance_add_dft(fdtd_ctx *c, int nparts, double *const *parts, const long long *lens);
+// The transforms' sums since the last read added into `parts` (doubles, interleaved, laid end to
+// end in the layout of fdtd_read_dft; lens: each part's), the device's then zero. Does nothing
+// where no step has been taken since the last read. wide: a long read may be added by an OpenMP team;
+// not in a thread that ends with the read, which would make and drop one.
+int fdtd_instance_add_dft(fdtd_ctx *c, int nparts, double *const *parts, const long long *lens, bool wide);
 int fdtd_instance_fail(fdtd_ctx *c, int code, const char *what);

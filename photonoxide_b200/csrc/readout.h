@@ -13,8 +13,8 @@ constexpr long long CHUNK = 1LL << 18;  // doubles: 2 MiB
 // chunk that was fetched whole; clear(count): starts the clearing of the first `count` doubles at the source.
 // fetch, wait and clear return 0 or an error. What has been added is cleared, on an error too, so that a
 // second read takes the rest and nothing twice; *taken, kept by the caller between reads, is how many doubles
-// have been added and could not be cleared. (One clearing a read: with one a chunk
-// a read of 161 MB took 12.7 ms, with one 11.3 to 12.6.)
+// have been added and could not be cleared. (One clearing a read: with one a chunk a
+// read of 161 MB took 12.7 ms, with one 11.3 to 12.6.)
 template <typename Fetch, typename Wait, typename Add, typename Clear>
 int read_add(long long n, long long *taken, double *const buffer[2], Fetch fetch, Wait wait, Add add,
              Clear clear) {

@@ -73,3 +73,28 @@ def test_a_job_without_its_fields_keeps_its_transforms():
             job.sim.e(0)
         with pytest.raises(GpuError):
             job.sim.run(1)
+
+
+def test_jobs_of_long_transforms():
+    """Whole-plane transforms of more than 2^19 doubles, several jobs read back at once."""
+    from photonoxide_b200.configs import N_SI
+    from photonoxide_b200.fdtd import Simulation
+    from photonoxide_b200.types import (INF, Axis, Boundaries, Boxes, Field, Grid3d, Source, Waveform)
+
+    def make(k):
+        g = Grid3d.centred((300, 301, 1), 0.02)
+        s = Simulation(g, Boxes(1.0).add((-INF, -0.1 - 0.05 * k, -INF), (INF, 0.2, INF), N_SI ** 2),
+                       Boundaries.cpml_2d(8), 0.5)
+        s.add_source(Source(Field.H, Axis.Z, (30, 150, 0), Waveform.pulse(1.0 / 1.55, 0.6)))
+        s.add_dft((0, 0, 0), (299, 300, 0), [1.0 / 1.55])
+        return s
+
+    alone = [make(k) for k in range(4)]
+    for s in alone:
+        s.run(90)
+    with Server(hbm_budget=2e9, max_active=4, chunk=64) as server:
+        jobs = [server.submit(make(k), 90, keep_fields=False) for k in range(4)]
+        for j, s in zip(jobs, alone):
+            assert j.wait() == DONE
+            sums = j.sim.transforms()
+            assert sums.size * 2 > 1 << 19 and np.array_equal(sums, s.transforms())
