@@ -28,6 +28,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <memory>
 #include <unordered_map>
 #include <vector>
 
@@ -2507,8 +2508,11 @@ struct fdtd_ctx {
   // first such transfer and kept (counted in the HBM budget)
   double *stage = nullptr;
   long long stage_len = 0;
-  // page-locked chunks the transforms' sums are read through, two in turn, made on the first large
-  // read and kept (fdtd_instance_add_dft); sums_fresh: steps have been taken since the last read
+  // the chunks the transforms' sums are read through (fdtd_instance_add_dft), made on first use and kept:
+  // plain memory, then two page-locked ones in turn; the doubles read so far; sums_fresh: steps have been
+  // taken since the last read
+  std::unique_ptr<double[]> plain;
+  long long plain_len = 0, sums_read = 0;
   double *host_stage[2] = {nullptr, nullptr};
   bool sums_fresh = true;
   long long sums_taken = 0;  // doubles of the sums read and not cleared (pxr::read_add)
@@ -4336,6 +4340,11 @@ void add_into_parts(const double *src, long long at, long long n, int nparts, do
 }
 }  // namespace
 
+// A context's reads go through page-locked memory once they come to more doubles than this in all (8 MiB).
+// The two chunks cost 4 to 6 ms to make and as much as that again to free, which a simulation run and read
+// once, or read little, never gets back: the first read of 49 000 doubles took 0.5 ms before there were any
+// and 6.2 with them, a repeated one 0.41 and 0.11.
+constexpr long long PINNED_READS = 1 << 20;
 // Read in 2 MiB chunks through two page-locked buffers, one filled while the other is added: a
 // whole-plane transform (400 x 200, six components, 21 frequencies: 161 MB) had gone through three
 // pageable arrays made for each read, twice a call.
@@ -4347,9 +4356,9 @@ int fdtd_instance_add_dft(fdtd_ctx *c, int nparts, double *const *parts, const l
   for (int p = 0; p < nparts; p++) room += lens[p];
   if (room != n) return fail(c, FDTD_E_INVALID, "the transforms hold %lld sums, not %lld", c->nsums, room / 2);
   if (n == 0 || !c->sums_fresh) return 0;
-  std::vector<double> plain;  // short reads, and where page-locked memory is refused
   double *buf[2] = {nullptr, nullptr};
-  if (n > CHUNK / 8) {
+  c->sums_read += n;
+  if (c->sums_read > PINNED_READS) {
     for (int b = 0; b < 2; b++)
       if (!c->host_stage[b] &&
           cudaHostAlloc((void **)&c->host_stage[b], CHUNK * 8, cudaHostAllocDefault) != cudaSuccess) {
@@ -4359,10 +4368,14 @@ int fdtd_instance_add_dft(fdtd_ctx *c, int nparts, double *const *parts, const l
     buf[0] = c->host_stage[0];
     buf[1] = c->host_stage[1];
   }
-  if (!buf[0] || !buf[1]) {
-    plain.resize(2 * std::min(n, CHUNK));
-    buf[0] = plain.data();
-    buf[1] = plain.data() + plain.size() / 2;
+  if (!buf[0] || !buf[1]) {  // plain memory, not paged in by more than the read
+    const long long each = std::min(n, CHUNK), want = n > CHUNK ? 2 * each : each;
+    if (c->plain_len < want) {
+      c->plain.reset(new double[want]);
+      c->plain_len = want;
+    }
+    buf[0] = c->plain.get();
+    buf[1] = buf[0] + (want - each);
   }
   auto fetch = [&](long long at, long long m, double *to) -> int {
     CUDA_TRY(c, cudaMemcpyAsync(to, c->sums + at, m * 8, cudaMemcpyDeviceToHost, c->stream));
