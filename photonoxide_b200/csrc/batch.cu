@@ -16,7 +16,7 @@
 // the grids' tiles; a tile computes H_z over itself and the row and column below it (its neighbours
 // compute the same values), adds the magnetic sources there, then updates E_x and E_y on its cells,
 // adds the electric sources, and writes both to the other copy of the fields.
-// Steps run in chunks of G: the source waveforms and transform phases of a chunk are evaluated
+// Steps run in chunks of G (or fewer): the source waveforms and transform phases of a chunk are evaluated
 // first (f64, the reference's exp and sincos), the chunk's step launches follow, the monitored
 // values copied into a ring as they go; at the chunk's end one launch adds the ring into the f64
 // transform sums in time order. A chunk is captured once as a CUDA graph and replayed.
@@ -28,6 +28,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <new>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -928,6 +929,8 @@ struct fdtd_batch {
   long long launches = 0;
   int sms = 148;
   std::vector<void *> allocs;  // this run's tables
+  size_t held = 0, room = SIZE_MAX;  // their bytes, and the most they may take (a context's own batch)
+  int chunk = G;                     // steps per chunk: G, or 16 where the ring has room for no more
   cudaGraphExec_t graph = nullptr;
   // the current tables (rebuilt at each run)
   void *d_insts = nullptr;
@@ -950,7 +953,7 @@ struct fdtd_batch {
   double *d_waves_h = nullptr, *d_waves_e = nullptr, *d_phase = nullptr;
   RecItem *d_rec = nullptr;
   long long nrec = 0;
-  void *d_ring = nullptr;  // G rows of the transform values
+  void *d_ring = nullptr;  // `chunk` rows of the transform values
   long long nring = 0;
   int blocks = 0;
   int *d_flags = nullptr;  // one TE-check flag per member
@@ -1001,6 +1004,7 @@ void free_tables(fdtd_batch *b) {
   b->graph = nullptr;
   for (void *p : b->allocs) cudaFreeAsync(p, b->stream);  // after the batch's work so far
   b->allocs.clear();
+  b->held = 0;
 }
 
 // Whether the batch can step simulation i (a 2D TE grid in the batch's precision, no media).
@@ -1020,13 +1024,24 @@ int admissible(fdtd_batch *b, const InstanceView &v, int i) {
   return 0;
 }
 
-template <typename V>
-int upload_vec(fdtd_batch *b, V **dst, const std::vector<V> &v) {
+// Device memory for one of the tables.
+int table(fdtd_batch *b, void **dst, size_t bytes) {
   *dst = nullptr;
-  size_t bytes = std::max<size_t>(v.size(), 1) * sizeof(V);
+  bytes = std::max<size_t>(bytes, 16);
+  if (bytes > b->room || b->held > b->room - bytes)
+    return bfail(b, FDTD_E_BUDGET, "the tables would exceed the HBM budget");
   void *p = nullptr;
   BTRY(b, cudaMallocAsync(&p, bytes, b->stream));  // stream-ordered: no device-wide sync
   b->allocs.push_back(p);
+  b->held += bytes;
+  *dst = p;
+  return 0;
+}
+template <typename V>
+int upload_vec(fdtd_batch *b, V **dst, const std::vector<V> &v) {
+  *dst = nullptr;
+  void *p = nullptr;
+  if (int r = table(b, &p, v.size() * sizeof(V))) return r;
   if (!v.empty())
     BTRY(b, cudaMemcpyAsync(p, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, b->stream));
   *dst = static_cast<V *>(p);
@@ -1034,8 +1049,7 @@ int upload_vec(fdtd_batch *b, V **dst, const std::vector<V> &v) {
 }
 int zeros(fdtd_batch *b, double **dst, size_t n) {
   void *p = nullptr;
-  BTRY(b, cudaMallocAsync(&p, std::max<size_t>(n, 1) * 8, b->stream));
-  b->allocs.push_back(p);
+  if (int r = table(b, &p, n * 8)) return r;
   BTRY(b, cudaMemsetAsync(p, 0, std::max<size_t>(n, 1) * 8, b->stream));
   *dst = static_cast<double *>(p);
   return 0;
@@ -1245,8 +1259,7 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
       // the recorded and the design's values by tile, each in the tile that owns its place
       const size_t E = sizeof(T);
       void *second = nullptr;
-      BTRY(b, cudaMallocAsync(&second, std::max<size_t>(v.psi_e_len, 1) * E, b->stream));
-      b->allocs.push_back(second);
+      if (int r = table(b, &second, v.psi_e_len * E)) return r;
       // what the tiles don't step there (E_z's psi, the rows' padding) is the engine's, so that either
       // copy may be handed back whole
       if (v.psi_e_len > 0)
@@ -1336,7 +1349,14 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
   if (int r = zeros(b, &b->d_waves_e, (size_t)G * std::max(b->nwaves_total, 1) * 2)) return r;
   if (int r = zeros(b, &b->d_phase, (size_t)G * std::max(b->nslots_total, 1) * 2)) return r;
   b->nring = nring;
-  {
+  b->chunk = G;
+  if (b->solo) {  // the engine's own ring, of as many rows as its memory rule allows
+    const InstanceView &v = views[0];
+    const long long rows = nring > 0 ? v.ring_k * v.nvalues / nring : G;
+    if (rows < 16) return bfail(b, FDTD_E_BUDGET, "the transforms' ring is too short for a chunk");
+    if (rows < G) b->chunk = 16;
+    b->d_ring = v.ring;
+  } else {
     double *ring = nullptr;
     if (int r = zeros(b, &ring, ((size_t)G * std::max<long long>(nring, 1) * sizeof(T) + 7) / 8))
       return r;
@@ -1432,7 +1452,7 @@ int occupancy(fdtd_batch *b) {
   return std::max(per, 1);
 }
 
-// `count` (<= G) steps of the current tables on the batch's stream; then the instances advance.
+// `count` (<= the chunk) steps of the current tables on the batch's stream; then the instances advance.
 // Returns how often the current copy has changed.
 template <typename T>
 int enqueue(fdtd_batch *b, int count) {
@@ -1498,14 +1518,15 @@ int finish_run(fdtd_batch *b, int64_t steps, const std::vector<InstanceView> &vi
   const int n = (int)b->ctxs.size();
   int64_t done = 0;
   *flips = 0;  // whole chunks are an even number of changes
-  const int64_t full = (steps - done) / G;
+  const int chunk = b->chunk;
+  const int64_t full = (steps - done) / chunk;
   if (full > 0) {
     if (!b->graph) {
       // one chunk captured as a graph, replayed
       cudaGraph_t g = nullptr;
       const long long before = b->launches;
       BTRY(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-      enqueue<T>(b, G);
+      enqueue<T>(b, chunk);
       cudaError_t err = cudaStreamEndCapture(b->stream, &g);
       if (err != cudaSuccess)
         return bfail(b, FDTD_E_GPU, "cudaStreamEndCapture: %s", cudaGetErrorString(err));
@@ -1520,9 +1541,9 @@ int finish_run(fdtd_batch *b, int64_t steps, const std::vector<InstanceView> &vi
       BTRY(b, cudaGraphLaunch(b->graph, b->stream));
       b->launches += b->per_chunk;
     }
-    done += full * G;
+    done += full * chunk;
   }
-  if (done < steps) *flips = enqueue<T>(b, (int)(steps - done));
+  if (done < steps) *flips = enqueue<T>(b, (int)(steps - done));  // fewer than a chunk
   BTRY(b, cudaGetLastError());
   if (SHAPES[b->shape].halo > 0) {
     // E's psi ends where the engine keeps it
@@ -1697,7 +1718,7 @@ int run_impl(fdtd_batch *b, int64_t steps, const int64_t *first_steps) {
 
 // A context's own run on the TE tiles (fdtd_solo_run).
 template <typename T>
-int solo_run(fdtd_batch *b, bool check, int64_t steps, int64_t first, bool *te) {
+int solo_run(fdtd_batch *b, bool check, int64_t steps, int64_t first, double *rows, bool *te) {
   std::vector<InstanceView> views(1);
   InstanceView &v = views[0];
   if (int r = fdtd_instance_view(b->ctxs[0], &v)) return r;
@@ -1734,8 +1755,6 @@ int solo_run(fdtd_batch *b, bool check, int64_t steps, int64_t first, bool *te) 
     if (bad) return 0;
     if (int r = settle_tm<T>(b, v)) return r;
   }
-  double *rows = nullptr;
-  if (int r = fdtd_instance_reserve(b->ctxs[0], steps, &rows)) return r;
   if (!b->reusable || b->solo_layout != v.layout) {
     b->reusable = false;
     b->aux = v.naux > 0;
@@ -1756,7 +1775,7 @@ int solo_run(fdtd_batch *b, bool check, int64_t steps, int64_t first, bool *te) 
 }  // namespace
 
 int fdtd_solo_run(fdtd_batch **batch, fdtd_ctx *ctx, bool check, int64_t steps, int64_t first,
-                  bool *te, long long *launches) {
+                  double *rows, size_t room, size_t *held, bool *te, long long *launches) {
   if (!*batch) {
     InstanceView v;
     if (int r = fdtd_instance_view(ctx, &v)) return r;
@@ -1772,9 +1791,16 @@ int fdtd_solo_run(fdtd_batch **batch, fdtd_ctx *ctx, bool check, int64_t steps, 
   }
   fdtd_batch *b = *batch;
   const long long before = b->launches;
-  const int r = b->precision == 64 ? solo_run<double>(b, check, steps, first, te)
-                                   : solo_run<float>(b, check, steps, first, te);
+  b->room = room;
+  int r = 0;
+  try {
+    r = b->precision == 64 ? solo_run<double>(b, check, steps, first, rows, te)
+                           : solo_run<float>(b, check, steps, first, rows, te);
+  } catch (const std::bad_alloc &) {
+    r = bfail(b, FDTD_E_GPU, "no host memory for the tables");
+  }
   *launches += b->launches - before;
+  *held = b->held;
   return r;
 }
 

@@ -2462,7 +2462,8 @@ struct fdtd_ctx {
   // last look at the fields found (1 TE, -1 not; 0: not looked at, or written by others than the engine's
   // steps of TE sources since)
   fdtd_batch *solo = nullptr;
-  bool solo_off = false;
+  size_t solo_held = 0;  // the bytes of its tables, in `used` too
+  unsigned long long solo_refused = ~0ULL;  // the layout its tables had no room in
   int te = 0;
   bool forced = false;  // a kernel was asked for by name
   int stride() const { return nwaves + naux + nbloch; }
@@ -2542,14 +2543,29 @@ int fail(fdtd_ctx *c, int code, const char *fmt, ...) {
                   __LINE__);                                                                   \
   } while (0)
 
+// The TE tiles' tables given back: they may be made again, and anything else comes before them.
+void drop_solo(fdtd_ctx *c) {
+  if (!c->solo) return;
+  fdtd_batch_destroy(c->solo);
+  c->solo = nullptr;
+  c->used -= c->solo_held;
+  c->solo_held = 0;
+}
+
 int alloc(fdtd_ctx *c, void **p, size_t bytes) {
   bytes = std::max<size_t>(bytes, 16);
+  if (c->budget && c->used + bytes > c->budget) drop_solo(c);
   if (c->budget && c->used + bytes > c->budget)
     return fail(c, FDTD_E_BUDGET, "%zu MB more would exceed the HBM budget of %zu MB",
                 bytes >> 20, c->budget >> 20);
   // stream-ordered, so that engines made and freed while others run (a serving loop) don't
   // synchronize the device; the stream's work so far is waited for before the memory is used
   cudaError_t e = cudaMallocAsync(p, bytes, c->stream);
+  if (e == cudaErrorMemoryAllocation && c->solo) {
+    cudaGetLastError();
+    drop_solo(c);
+    e = cudaMallocAsync(p, bytes, c->stream);
+  }
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -2934,16 +2950,12 @@ void launch_aux(fdtd_ctx *c, int stride, long long first, const long long *base,
 // sources on E_x, E_y and H_z alone, none of the parts the tiles don't step, and enough steps to
 // pay for looking the fields up (about 25 us a run, against 10 us a step on the quad kernel).
 bool solo_ok(const fdtd_ctx *c, long long steps) {
-  if (c->solo_off || c->forced || c->profiling || c->capturing || steps < SOLO_STEPS || c->te < 0) return false;
+  if (c->solo_refused == c->layout || c->forced || c->profiling || c->capturing || steps < SOLO_STEPS || c->te < 0) return false;
   if (c->n[2] != 1 || !c->periodic[2] || c->media || c->nbloch > 0) return false;
   if (c->naux_runs > 0 && !c->aux_te) return false;
+  if (c->nvalues > 0 && c->ring_k < 8) return false;  // no ring of a chunk's steps (fdtd_batch::chunk)
   for (const fdtd_injection &x : c->src_inj)
     if ((x.field == 1) != (x.component == 2) && x.point != 2) return false;
-  if (c->budget) {
-    // E's psi again, and per monitored value its record, item and 32 steps
-    const size_t more = c->psi_e_len * c->elem + (size_t)c->nvalues * (64 + 32 * c->elem) + (1u << 20);
-    if (c->used + more > c->budget) return false;
-  }
   return true;
 }
 
@@ -2958,16 +2970,21 @@ int run_impl(fdtd_ctx *c, long long steps, long long first) {
   c->sums_fresh = true;
   if (solo_ok(c, steps)) {
     bool te = false;
-    const int r = fdtd_solo_run(&c->solo, c, c->te == 0, steps, first, &te, &c->launches);
+    double *rows = nullptr;
+    if (int r = fdtd_instance_reserve(c, steps, &rows)) return r;
+    const size_t room = c->budget ? c->budget - std::min(c->budget, c->used - c->solo_held) : SIZE_MAX;
+    size_t held = 0;
+    const int r = fdtd_solo_run(&c->solo, c, c->te == 0, steps, first, rows, room, &held, &te, &c->launches);
+    c->used += held - c->solo_held;
+    c->solo_held = held;
     if (te) {
       c->te = 1;
       return r == 0 ? 0 : fail(c, r, "a run on the TE tiles: %s", fdtd_batch_last_error(c->solo));
     }
     if (r) {  // no room for its tables: nothing has run, and the general path serves
       cudaGetLastError();
-      fdtd_batch_destroy(c->solo);
-      c->solo = nullptr;
-      c->solo_off = true;
+      drop_solo(c);
+      c->solo_refused = c->layout;
     } else {
       c->te = -1;  // looked at once, not on each run
     }
@@ -4276,6 +4293,8 @@ int fdtd_instance_view(fdtd_ctx *c, InstanceView *v) {
   v->slot_field = c->d_slot_field;
   v->sums = c->sums;
   v->nsums = c->nvalues > 0 ? c->nsums : 0;
+  v->ring = c->ring;
+  v->ring_k = c->ring_k;
   v->freq_chunks = c->freq_chunks;
   v->nprobes = c->nprobes;
   v->probes = c->d_probes;

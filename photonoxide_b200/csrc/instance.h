@@ -34,6 +34,8 @@ struct InstanceView {
   const int *slot_field;
   double *sums;
   long long nsums;  // complex sums
+  void *ring;  // the transforms' ring: ring_k rows of nvalues
+  int ring_k;
   int freq_chunks;  // the most frequencies of a series, in chunks of DFT_F (at least 1)
   int nprobes;
   const long long *probes;
@@ -58,10 +60,12 @@ int fdtd_instance_aux(fdtd_ctx *c, int stride, const long long *base, int count,
 // A 2D TE context's own steps on the batch's tiles of several steps a launch, enqueued on its stream
 // (batch.cu). *batch: made on the first call, the context's to destroy. check: whether the fields may
 // have come from elsewhere since the last such run: that H_x, H_y, E_z are zero is then looked up
-// (and waited for); *te false: they are not, and nothing has run. Adds its launches to *launches.
+// (and waited for); *te false: they are not, or it returns an error (its tables would take more than
+// `room` bytes, or there is no memory for them), and nothing has run. rows: the probe record's (reserved);
+// *held: the bytes its tables take. Adds its launches to *launches.
 struct fdtd_batch;
 int fdtd_solo_run(fdtd_batch **batch, fdtd_ctx *c, bool check, int64_t steps, int64_t first,
-                  bool *te, long long *launches);
+                  double *rows, size_t room, size_t *held, bool *te, long long *launches);
 // The transforms' sums since the last read added into `parts` (doubles, interleaved, laid end to
 // end in the layout of fdtd_read_dft; lens: each part's), the device's then zero. Does nothing
 // where no step has been taken since the last read. wide: a long read may be added by an OpenMP team;
