@@ -29,13 +29,14 @@ int fdtd_batch_create(int32_t count, fdtd_ctx *const *ctxs, fdtd_batch **out);
 const char *fdtd_batch_last_error(const fdtd_batch *batch);
 /* `steps` steps of every grid; grid i's first step has index first_steps[i] (its step count so
  * far, as fdtd_run's first_step), all 0 when first_steps is NULL. A batch whose tile shape is not set
- * takes one by its size, of several steps a launch but for few cells in f64. Returns
+ * takes one on its first run: by the grids' sizes where they tell, else the fastest of all shapes, each
+ * timed on 32 of the run's steps when it has 320 or more. Returns
  * once the steps are queued: each context's stream waits for them, so its later calls (reads,
  * runs, fdtd_synchronize) come after. */
 int fdtd_batch_run(fdtd_batch *batch, int64_t steps, const int64_t *first_steps);
 /* The tile shape in use (0 x 0 before the first run chooses one). */
 int fdtd_batch_tile(const fdtd_batch *batch, int32_t *width, int32_t *height);
-/* Fixes the tile shape, or 0 x 0: by the batch's size on the next run. One step a launch: 32x8,
+/* Fixes the tile shape, or 0 x 0: chosen on the next run. One step a launch: 32x8,
  * 32x16, 64x4, 64x8, 128x2, 128x4, or 124x7 (a warp per row of 124 places, four a lane). Several:
  * 112x16 (eight steps), 120x40 in f32 and 120x24 in f64 (four). */
 int fdtd_batch_set_tile(fdtd_batch *batch, int32_t width, int32_t height);

@@ -70,10 +70,12 @@ class Batch:
         raise GpuError(msg)
 
     def run(self, steps: int) -> "Batch":
-        """``steps`` steps of every simulation. A batch without a fixed tile shape takes tiles of
-        several steps a launch: in f32 112x16 (eight steps) for few cells, 120x40 (four) for many;
-        in f64 120x24 (four) for many and 64x8 (one) for few. The shapes of one step a launch are
-        32x8, 32x16, 64x4, 64x8, 128x2, 128x4 and the 124x7 rows."""
+        """``steps`` steps of every simulation. A batch without a fixed tile shape chooses one on its
+        first run: tiles of several steps a launch where the grids fill them (in f32 112x16, eight
+        steps, for few cells and 120x40, four, for many; in f64 120x24, four, for many); where the
+        sizes do not tell, the fastest of all shapes, each timed on 32 of the run's steps when it
+        has 320 or more. The shapes of one step a launch are 32x8, 32x16, 64x4, 64x8, 128x2, 128x4
+        and the 124x7 rows."""
         self._check(_lib().pxs_batch_run(self._h, int(steps)))
         return self
 

@@ -907,7 +907,7 @@ struct Shape {
 // taller tile's values have no registers, 120 x 40 in f32)
 const Shape SHAPES[] = {{32, 8, 0}, {32, 16, 0}, {64, 4, 0}, {64, 8, 0}, {128, 2, 0}, {128, 4, 0},
                         {teq::OWN, teq::RW, 0}, {112, 16, 8}, {120, 24, 4}, {120, 40, 4}};
-constexpr int ONE_STEP = 3, QUAD_SHAPE = 6, BLOCK_SMALL = 7, BLOCK_LARGE = 8, BLOCK_TALL = 9;
+constexpr int ONE_STEP_NARROW = 1, ONE_STEP = 3, QUAD_SHAPE = 6, BLOCK_SMALL = 7, BLOCK_LARGE = 8, BLOCK_TALL = 9;
 constexpr int NSHAPES = sizeof(SHAPES) / sizeof(SHAPES[0]);
 // te_block_kernel's warps: f32, 16 of 2 rows (eight steps a launch) or 3 (four: fewer halo places);
 // f64, 8 of 4 rows.
@@ -925,7 +925,8 @@ struct fdtd_batch {
   int precision = 32;
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr, t0 = nullptr, t1 = nullptr;
-  int shape = -1;  // index into SHAPES; -1: by the size on the next run (block_shape)
+  int shape = -1;  // index into SHAPES; -1: chosen on the next run (choose_shape)
+  bool trial = true;  // whether that run may time the shapes
   long long launches = 0;
   int sms = 148;
   std::vector<void *> allocs;  // this run's tables
@@ -1511,13 +1512,26 @@ int enqueue(fdtd_batch *b, int count) {
   return flips;
 }
 
+// After `flips` changes of the current copies E's psi goes where the engine keeps it.
+template <typename T>
+int hand_back(fdtd_batch *b, const std::vector<InstanceView> &views, int flips) {
+  if (SHAPES[b->shape].halo == 0) return 0;
+  b->psi_flips = (b->psi_flips + flips) & 1;
+  for (size_t i = 0; i < views.size() && b->psi_flips; i++)
+    if (views[i].psi_e_len > 0)
+      BTRY(b, cudaMemcpyAsync(views[i].psi_e, b->psi2[i], views[i].psi_e_len * sizeof(T),
+                              cudaMemcpyDeviceToDevice, b->stream));
+  return 0;
+}
+
 // The run's steps from `done` on with the current tables: whole chunks by the captured graph
 // (captured now if there is none), the rest launched; then the members' streams wait for them.
+// *flips: the changes of the current copies so far, these steps' added.
 template <typename T>
-int finish_run(fdtd_batch *b, int64_t steps, const std::vector<InstanceView> &views, int *flips) {
+int finish_run(fdtd_batch *b, int64_t steps, int64_t done, const std::vector<InstanceView> &views,
+               int *flips) {
   const int n = (int)b->ctxs.size();
-  int64_t done = 0;
-  *flips = 0;  // whole chunks are an even number of changes
+  int last = 0;  // whole chunks are an even number of changes
   const int chunk = b->chunk;
   const int64_t full = (steps - done) / chunk;
   if (full > 0) {
@@ -1543,17 +1557,10 @@ int finish_run(fdtd_batch *b, int64_t steps, const std::vector<InstanceView> &vi
     }
     done += full * chunk;
   }
-  if (done < steps) *flips = enqueue<T>(b, (int)(steps - done));  // fewer than a chunk
+  if (done < steps) last = enqueue<T>(b, (int)(steps - done));  // fewer than a chunk
   BTRY(b, cudaGetLastError());
-  if (SHAPES[b->shape].halo > 0) {
-    // E's psi ends where the engine keeps it
-    b->psi_flips = (b->psi_flips + *flips) & 1;
-    if (b->psi_flips)
-      for (int i = 0; i < n; i++)
-        if (views[i].psi_e_len > 0)
-          BTRY(b, cudaMemcpyAsync(views[i].psi_e, b->psi2[i], views[i].psi_e_len * sizeof(T),
-                                  cudaMemcpyDeviceToDevice, b->stream));
-  }
+  if (int r = hand_back<T>(b, views, last)) return r;
+  *flips += last;
   if (!b->solo) BTRY(b, cudaEventRecord(b->done, b->stream));
   for (int i = 0; i < n; i++) {
     if (!b->solo) BTRY(b, cudaStreamWaitEvent(views[i].stream, b->done, 0));
@@ -1564,26 +1571,55 @@ int finish_run(fdtd_batch *b, int64_t steps, const std::vector<InstanceView> &vi
   return 0;
 }
 
-// The tile shape of a batch whose caller fixed none. f32: te_block_kernel's, eight steps a launch while
-// its tiles fill the SMs a few times over, four steps beyond (us a step, eight against four: one
-// 537 x 541 grid 6.6 and 9.2; 1.29 M cells in six 17.7 and 17.9; 2.6 M in twelve 33.1 and 32.0; 19.2 M
-// in 64 212 and 186; one step a launch 12.2, 30.6, 54.2 and 374). f64, where a tile has half the warps:
-// four steps a launch from about 1.3 M cells on (40.2 us against one step's 40.2; 3.4 M cells 85.5 and
-// 98.9, 10.4 M 209 and 266), one step below (0.16 M cells 16.9 and 11.4).
-int block_shape(const std::vector<InstanceView> &views, int sms, bool one_step) {
-  auto tiles = [&](int shape) {
-    long long n = 0;
-    for (const InstanceView &v : views)
-      n += (long long)((v.n[0] + SHAPES[shape].tw - 1) / SHAPES[shape].tw) *
-           ((v.n[1] + SHAPES[shape].th - 1) / SHAPES[shape].th);
-    return n;
-  };
-  if (views[0].precision == 64) {
-    if (one_step && tiles(BLOCK_LARGE) <= 4LL * sms) return ONE_STEP;
-    return tiles(BLOCK_SMALL) <= sms ? BLOCK_SMALL : BLOCK_LARGE;
+// The share of the tiles' own places that are the grids'.
+double fill(const std::vector<InstanceView> &views, int shape) {
+  double cells = 0.0, places = 0.0;
+  for (const InstanceView &v : views) {
+    const int tw = SHAPES[shape].tw, th = SHAPES[shape].th;
+    cells += (double)v.n[0] * v.n[1];
+    places += (double)((v.n[0] + tw - 1) / tw) * ((v.n[1] + th - 1) / th) * tw * th;
   }
-  return tiles(BLOCK_SMALL) <= 6LL * sms ? BLOCK_SMALL : BLOCK_TALL;
+  return cells / places;
 }
+long long count_tiles(const std::vector<InstanceView> &views, int shape) {
+  long long n = 0;
+  for (const InstanceView &v : views)
+    n += (long long)((v.n[0] + SHAPES[shape].tw - 1) / SHAPES[shape].tw) *
+         ((v.n[1] + SHAPES[shape].th - 1) / SHAPES[shape].th);
+  return n;
+}
+
+// The tiles of several steps a launch for these grids. f32: eight steps while the tiles fill the SMs a few
+// times over, four beyond (us a step, eight against four: one 537 x 541 grid 6.6 and 9.2; 1.29 M cells in six
+// 17.7 and 17.9; 2.6 M in twelve 33.1 and 32.0; 19.2 M in 64 212 and 186; one step a launch 12.2, 30.6, 54.2
+// and 374). f64, where a tile has half the warps: four steps but for grids of a tile an SM or fewer.
+int block_shape(const std::vector<InstanceView> &views, int sms) {
+  if (views[0].precision == 64)
+    return count_tiles(views, BLOCK_SMALL) <= sms ? BLOCK_SMALL : BLOCK_LARGE;
+  return count_tiles(views, BLOCK_SMALL) <= 6LL * sms ? BLOCK_SMALL : BLOCK_TALL;
+}
+
+// The tile shape of a batch whose caller fixed none; *sure: whether sizes alone tell, or the shapes had better
+// be timed. Sizes tell in f32 where the tiles of several steps are few (up to two an SM a step is its launches:
+// 16 grids of 64 x 64 5.0 us a step and 6.7 with the best of one step) or at least 65 % full (256 grids of
+// 100 x 100, 69 %: 53 and 70), and in f64 where more than four an SM are at least 85 % full (above: 10.4 M cells
+// in 35 209 and 266). Between, either may be the faster by half: f32, 256 grids of 64 x 64, 43 % full, 37 against
+// 28, of 136 x 136, 48 %, 115 against 130; f64, 256 of 100 x 100, 69 %, 145 against 111, 1024 of 32 x 32 272
+// against 49; f64 and small, 64 grids and fewer, which one-step shape is best changes too.
+int choose_shape(const std::vector<InstanceView> &views, int sms, bool *sure) {
+  const int block = block_shape(views, sms);
+  if (views[0].precision == 64) {
+    *sure = count_tiles(views, BLOCK_LARGE) > 4LL * sms && fill(views, BLOCK_LARGE) >= 0.85;
+    if (*sure) return BLOCK_LARGE;
+    return fill(views, ONE_STEP) >= 0.8 ? ONE_STEP : ONE_STEP_NARROW;
+  }
+  *sure = count_tiles(views, BLOCK_SMALL) <= 2LL * sms || fill(views, block) >= 0.65;
+  return *sure || fill(views, block) >= 0.5 ? block : ONE_STEP_NARROW;
+}
+// Steps a shape is timed on, after as many untimed (an even number of launches of any shape), and the
+// shortest run that times them: nine shapes in f32, nine in f64, and a chunk.
+constexpr int TRIAL = 16;
+constexpr int TRIAL_STEPS = 2 * TRIAL * (NSHAPES - 1) + G;
 
 // A run whose members are all as the last run left them: its tables and graph serve again, the
 // members' streams ordered before it by events (no host waits, no checks, no rebuild).
@@ -1611,7 +1647,7 @@ int run_again(fdtd_batch *b, int64_t steps, const int64_t *first_steps, bool *ra
     BTRY(b, cudaStreamWaitEvent(b->stream, b->member_ev[i], 0));
   }
   int flips = 0;
-  if (int r = finish_run<T>(b, steps, views, &flips)) return r;
+  if (int r = finish_run<T>(b, steps, 0, views, &flips)) return r;
   for (int i = 0; i < n; i++) {
     b->next_first[i] += steps;
     b->next_parity[i] = (b->next_parity[i] + flips) & 1;
@@ -1696,13 +1732,52 @@ int run_impl(fdtd_batch *b, int64_t steps, const int64_t *first_steps) {
         return bfail(b, FDTD_E_INVALID,
                      "simulation %d has H_x, H_y or E_z values: the batch steps TE fields only", i);
   }
-  if (b->shape < 0) b->shape = block_shape(views, b->sms, true);
-  if (int r = build<T>(b, views, first, parity, rows, b->shape)) return r;
-  if (SHAPES[b->shape].halo > 0) launch_shape<T>(b, 0, 0, 0);
-  else b->blocks = occupancy<T>(b) * b->sms;
   b->reusable = false;
+  auto rebuild = [&](int shape) -> int {
+    if (int r = build<T>(b, views, first, parity, rows, shape)) return r;
+    if (SHAPES[shape].halo > 0) launch_shape<T>(b, 0, 0, 0);
+    else b->blocks = occupancy<T>(b) * b->sms;
+    return 0;
+  };
   int flips = 0;
-  if (int r = finish_run<T>(b, steps, views, &flips)) return r;
+  int64_t done = 0;
+  if (b->shape < 0) {
+    bool sure = false;
+    int pick = choose_shape(views, b->sms, &sure);
+    if (!sure && b->trial && b->record && b->ndesign == 0 && steps >= TRIAL_STEPS) {
+      float best = 1e30f;
+      for (int shape = 0; shape < NSHAPES; shape++) {
+        if (shape == (b->precision == 64 ? BLOCK_TALL : BLOCK_LARGE)) continue;
+        if (int r = rebuild(shape)) return r;
+        int took = enqueue<T>(b, TRIAL);
+        BTRY(b, cudaEventRecord(b->t0, b->stream));
+        took += enqueue<T>(b, TRIAL);
+        BTRY(b, cudaEventRecord(b->t1, b->stream));
+        if (int r = hand_back<T>(b, views, took)) return r;
+        // where the device's descriptors have moved the instances to
+        std::vector<TeInst<T>> now(n);
+        BTRY(b, cudaMemcpyAsync(now.data(), b->d_insts, n * sizeof(TeInst<T>), cudaMemcpyDeviceToHost,
+                                b->stream));
+        BTRY(b, cudaStreamSynchronize(b->stream));
+        for (int i = 0; i < n; i++) {
+          first[i] = now[i].first;
+          parity[i] = now[i].parity;
+          rows[i] = now[i].rows;
+        }
+        float ms = 0.f;
+        BTRY(b, cudaEventElapsedTime(&ms, b->t0, b->t1));
+        if (ms < best) {
+          best = ms;
+          pick = shape;
+        }
+        flips += took;
+        done += 2 * TRIAL;
+      }
+    }
+    b->shape = pick;
+  }
+  if (int r = rebuild(b->shape)) return r;
+  if (int r = finish_run<T>(b, steps, done, views, &flips)) return r;
   b->reusable = true;
   b->cap_record = b->record;
   b->gens.assign(n, 0);
@@ -1758,7 +1833,7 @@ int solo_run(fdtd_batch *b, bool check, int64_t steps, int64_t first, double *ro
   if (!b->reusable || b->solo_layout != v.layout) {
     b->reusable = false;
     b->aux = v.naux > 0;
-    b->shape = block_shape(views, b->sms, false);
+    b->shape = block_shape(views, b->sms);
     if (int r = build<T>(b, views, {first}, {v.parity}, {rows}, b->shape)) return r;
     launch_shape<T>(b, 0, 0, 0);
     b->solo_layout = v.layout;
@@ -1769,10 +1844,12 @@ int solo_run(fdtd_batch *b, bool check, int64_t steps, int64_t first, double *ro
   b->launches++;
   b->psi_flips = 0;
   int flips = 0;
-  return finish_run<T>(b, steps, views, &flips);
+  return finish_run<T>(b, steps, 0, views, &flips);
 }
 
 }  // namespace
+
+void fdtd_batch_no_trial(fdtd_batch *b) { b->trial = false; }
 
 int fdtd_solo_run(fdtd_batch **batch, fdtd_ctx *ctx, bool check, int64_t steps, int64_t first,
                   double *rows, size_t room, size_t *held, bool *te, long long *launches) {
@@ -2022,7 +2099,7 @@ int adjoint_tables(fdtd_adjoint *a, const InstanceView &v, const std::vector<lon
   int dev = 0, sms = 148;
   ATRY(a, cudaGetDevice(&dev));
   ATRY(a, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  a->shape = block_shape({v}, sms, false);
+  a->shape = block_shape({v}, sms);
   const int TW = SHAPES[a->shape].tw, TH = SHAPES[a->shape].th, halo = SHAPES[a->shape].halo;
   const int nx = v.n[0], ny = v.n[1];
   a->tiles_x = (nx + TW - 1) / TW;
@@ -2292,6 +2369,7 @@ int fdtd_adjoint_create(fdtd_ctx *ctx, int64_t steps, int32_t segment, int64_t c
   fdtd_ctx *one[1] = {ctx};
   if (int q = fdtd_batch_create(1, one, &a->batch))
     return afail(a, q, "%s", fdtd_batch_last_error(a->batch));
+  fdtd_batch_no_trial(a->batch);  // one grid, whose steps are all alike
   return 0;
 }
 

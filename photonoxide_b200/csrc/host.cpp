@@ -2779,6 +2779,7 @@ struct pxs_server {
             batch = nullptr;
             te.clear();
           } else {
+            fdtd_batch_no_trial(batch);  // remade whenever a job joins or ends
             batch_jobs = te;
           }
         }

@@ -57,13 +57,15 @@ void fdtd_instance_advance(fdtd_ctx *c, long long steps, int flips);
 // values into the tables of `stride` values a step after the emitters'; the kernels launched.
 int fdtd_instance_aux(fdtd_ctx *c, int stride, const long long *base, int count, double *out_h,
                       double *out_e);
+struct fdtd_batch;
+// The batch takes a tile shape by its size alone, without timing any: one that is remade often.
+void fdtd_batch_no_trial(fdtd_batch *batch);
 // A 2D TE context's own steps on the batch's tiles of several steps a launch, enqueued on its stream
 // (batch.cu). *batch: made on the first call, the context's to destroy. check: whether the fields may
 // have come from elsewhere since the last such run: that H_x, H_y, E_z are zero is then looked up
 // (and waited for); *te false: they are not, or it returns an error (its tables would take more than
 // `room` bytes, or there is no memory for them), and nothing has run. rows: the probe record's (reserved);
 // *held: the bytes its tables take. Adds its launches to *launches.
-struct fdtd_batch;
 int fdtd_solo_run(fdtd_batch **batch, fdtd_ctx *c, bool check, int64_t steps, int64_t first,
                   double *rows, size_t room, size_t *held, bool *te, long long *launches);
 // The transforms' sums since the last read added into `parts` (doubles, interleaved, laid end to

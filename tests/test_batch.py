@@ -80,7 +80,7 @@ CASES4 = [
 
 @pytest.mark.parametrize("precision", [32, 64])
 def test_batch_matches_the_oracle_and_each_grid_alone(precision):
-    """500 steps: the first run times the seven tile shapes on 448 of them."""
+    """500 steps: in f64 the first run times the tile shapes on 288 of them."""
     batch = [te_busy(Simulation, n, b, 100 * i, precision) for i, (n, b) in enumerate(CASES)]
     alone = [te_busy(Simulation, n, b, 100 * i, precision) for i, (n, b) in enumerate(CASES)]
     oracle = [te_busy(OracleSimulation, n, b, 100 * i, precision) for i, (n, b) in enumerate(CASES)]

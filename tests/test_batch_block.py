@@ -79,3 +79,20 @@ def test_a_te_run_alone_takes_the_same_tiles(precision):
         s.set_field(Field.E, Axis.Z, np.full(n[0] * n[1], 0.01))  # no longer TE
         s.run(40)
     same(a, o)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+def test_many_small_grids_time_the_shapes(precision):
+    """Grids that fill a third of a tile, too many for the tiles to be few: the first run of 320 steps or
+    more times every shape on steps of its own, with probes and transforms; a shorter one takes a shape
+    by the sizes. The bits of each grid alone."""
+    n, b = EDGES[0]
+    for steps in (330, 40):
+        a = [te_busy(Simulation, n, b, 5 * i, precision) for i in range(200)]
+        B = Batch(a)
+        B.run(steps)
+        B.run(21)
+        for i in (0, 77, 199):
+            o = te_busy(general, n, b, 5 * i, precision)
+            o.run(steps + 21)
+            same(a[i], o)
