@@ -627,12 +627,25 @@ __global__ void te_zero_kernel(ZeroRanges R, int *bad) {
     if (p[q] != T(0)) atomicOr(bad, 1);
 }
 
-// Nonzero values among H_x, H_y, E_z of the current copy (the batch steps TE grids only).
+// Nonzero values among H_x, H_y, E_z of the current copy (e, h, psi_h) set *bad: the tiles step TE grids
+// only. The other copy's (eo, ho, psi_ho) are set to zero, and its psi of H_x and H_y to the current one's:
+// either copy may end as the current one, and the other's psi is whatever the steps before an upload left
+// there.
+struct PsiRanges {
+  long long at[4], len[4];
+  int count;
+};
 template <typename T>
-__global__ void te_tm_check_kernel(const T *e, const T *h, long long N, int *bad) {
-  long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= N) return;
-  if (h[q] != T(0) || h[N + q] != T(0) || e[2 * N + q] != T(0)) atomicOr(bad, 1);
+__global__ void te_settle_kernel(const T *e, const T *h, const T *psi_h, T *eo, T *ho, T *psi_ho, long long N,
+                                 PsiRanges R, int *bad) {
+  const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < N) {
+    if (h[q] != T(0) || h[N + q] != T(0) || e[2 * N + q] != T(0)) atomicOr(bad, 1);
+    ho[q] = ho[N + q] = eo[2 * N + q] = T(0);
+  }
+  for (int r = 0; r < R.count; r++)
+    for (long long p = q; p < R.len[r]; p += (long long)gridDim.x * blockDim.x)
+      psi_ho[R.at[r] + p] = psi_h[R.at[r] + p];
 }
 
 // After step m of a chunk: the curl E's update multiplies by cb, at each design value (its
@@ -972,6 +985,9 @@ struct fdtd_batch {
   bool reusable = false;
   // a context's own batch of one, on its stream (fdtd_solo_run); aux: it has a plane wave's run
   bool solo = false, aux = false;
+  // the members' monitored values and probes as a run's tables need them, read from the device once a run
+  bool places_read = false;
+  std::vector<std::vector<long long>> where, probes;
   unsigned long long solo_layout = 0;
   bool cap_record = true;
   long long per_chunk = 0;  // the graph's kernels
@@ -1056,6 +1072,29 @@ int zeros(fdtd_batch *b, double **dst, size_t n) {
   return 0;
 }
 
+int read_places(fdtd_batch *b, const std::vector<InstanceView> &views) {
+  const size_t n = views.size();
+  b->where.assign(n, {});
+  b->probes.assign(n, {});
+  for (size_t i = 0; i < n; i++) {
+    const InstanceView &v = views[i];
+    b->where[i].resize(v.nvalues);
+    b->probes[i].resize(v.nprobes);
+    if (v.nvalues)
+      BTRY(b, cudaMemcpyAsync(b->where[i].data(), v.where, v.nvalues * 8, cudaMemcpyDeviceToHost, b->stream));
+    if (v.nprobes)
+      BTRY(b, cudaMemcpyAsync(b->probes[i].data(), v.probes, v.nprobes * 8, cudaMemcpyDeviceToHost, b->stream));
+  }
+  BTRY(b, cudaStreamSynchronize(b->stream));
+  b->places_read = true;
+  return 0;
+}
+void drop_places(fdtd_batch *b) {
+  b->places_read = false;
+  b->where.clear();
+  b->probes.clear();
+}
+
 // The tables for tile shape `sh`: per-instance descriptors (starting at step first[i], copy
 // parity[i], record row rows[i]), the tile list, the sources' groups per tile, the waveforms,
 // the transforms' phase slots and the record items.
@@ -1070,6 +1109,15 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
   std::vector<TeDesign> ditems;
   b->psi2.assign(views.size(), nullptr);
   b->psi_flips = 0;
+  void *psi2 = nullptr;  // the members' second copies, one after another
+  size_t psi2_at = 0;
+  if (halo > 0) {
+    size_t bytes = 0;
+    for (const InstanceView &v : views) bytes += (v.psi_e_len * sizeof(T) + 255) / 256 * 256;
+    if (int r = table(b, &psi2, bytes)) return r;
+    if (b->record && !b->places_read)
+      if (int r = read_places(b, views)) return r;
+  }
   std::vector<TeInst<T>> insts(views.size());
   std::vector<int> tile_inst;
   std::vector<int> hb{0}, eb{0};
@@ -1259,8 +1307,8 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
     } else {
       // the recorded and the design's values by tile, each in the tile that owns its place
       const size_t E = sizeof(T);
-      void *second = nullptr;
-      if (int r = table(b, &second, v.psi_e_len * E)) return r;
+      void *second = (char *)psi2 + psi2_at;
+      psi2_at += (v.psi_e_len * E + 255) / 256 * 256;
       // what the tiles don't step there (E_z's psi, the rows' padding) is the engine's, so that either
       // copy may be handed back whole
       if (v.psi_e_len > 0)
@@ -1284,12 +1332,7 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
         (it.comp == 2 ? hp : ep)[t].push_back(it);
       };
       if (b->record) {
-        std::vector<long long> where(v.nvalues), probes(v.nprobes);
-        if (v.nvalues)
-          BTRY(b, cudaMemcpyAsync(where.data(), v.where, v.nvalues * 8, cudaMemcpyDeviceToHost, b->stream));
-        if (v.nprobes)
-          BTRY(b, cudaMemcpyAsync(probes.data(), v.probes, v.nprobes * 8, cudaMemcpyDeviceToHost, b->stream));
-        BTRY(b, cudaStreamSynchronize(b->stream));
+        const std::vector<long long> &where = b->where[i], &probes = b->probes[i];
         for (long long q = 0; q < v.nvalues; q++) {
           const int comp = (int)((where[q] & ((1LL << 62) - 1)) / v.N);
           if ((where[q] >> 62 != 0) != (comp == 2)) continue;
@@ -1656,23 +1699,24 @@ int run_again(fdtd_batch *b, int64_t steps, const int64_t *first_steps, bool *ra
   return 0;
 }
 
-// The other copy's H_x, H_y and E_z, which the steps leave alone, as the current copy's are: the fields at
-// zero, H's psi the current one's. (Either copy may end as the current one, and the other's psi is whatever
-// the steps before an upload left there.)
+// The other copy's H_x, H_y and E_z, which the steps leave alone, made as the current copy's are
+// (te_settle_kernel); a nonzero field of them in the current copy sets *bad.
 template <typename T>
-int settle_tm(fdtd_batch *b, const InstanceView &v) {
-  const size_t E = sizeof(T);
-  const int other = 1 - v.parity;
-  BTRY(b, cudaMemsetAsync((char *)v.h[other], 0, 2 * v.N * E, b->stream));
-  BTRY(b, cudaMemsetAsync((char *)v.e[other] + 2 * v.N * E, 0, v.N * E, b->stream));
+int settle_tm(fdtd_batch *b, const InstanceView &v, int *bad) {
+  PsiRanges R;
+  R.count = 0;
   for (int axis = 0; axis < 2; axis++)  // H_y's slabs along x, H_x's along y
     for (int side = 0; side < 2; side++) {
       const SlabEntry &s = v.table[1][1 - axis][axis][side];
-      const size_t len = axis == 0 ? (size_t)s.pw * v.n[1] : (size_t)s.count * v.pitch;
-      if (s.count > 0)
-        BTRY(b, cudaMemcpyAsync((T *)v.psi_h[other] + s.psi, (const T *)v.psi_h[v.parity] + s.psi, len * E,
-                                cudaMemcpyDeviceToDevice, b->stream));
+      if (s.count == 0) continue;
+      R.at[R.count] = s.psi;
+      R.len[R.count++] = axis == 0 ? (long long)s.pw * v.n[1] : (long long)s.count * v.pitch;
     }
+  const int other = 1 - v.parity;
+  te_settle_kernel<T><<<(unsigned)((v.N + 255) / 256), 256, 0, b->stream>>>(
+      (const T *)v.e[v.parity], (const T *)v.h[v.parity], (const T *)v.psi_h[v.parity], (T *)v.e[other],
+      (T *)v.h[other], (T *)v.psi_h[other], v.N, R, bad);
+  BTRY(b, cudaGetLastError());
   return 0;
 }
 
@@ -1718,9 +1762,7 @@ int run_impl(fdtd_batch *b, int64_t steps, const int64_t *first_steps) {
     const InstanceView &v = views[i];
     BTRY(b, cudaEventRecord(b->member_ev[i], v.stream));
     BTRY(b, cudaStreamWaitEvent(b->stream, b->member_ev[i], 0));
-    te_tm_check_kernel<T><<<(unsigned)((v.N + 255) / 256), 256, 0, b->stream>>>(
-        (const T *)v.e[v.parity], (const T *)v.h[v.parity], v.N, b->d_flags + i);
-    if (int r = settle_tm<T>(b, v)) return r;
+    if (int r = settle_tm<T>(b, v, b->d_flags + i)) return r;
   }
   {
     std::vector<int> bad(n, 0);
@@ -1733,6 +1775,7 @@ int run_impl(fdtd_batch *b, int64_t steps, const int64_t *first_steps) {
                      "simulation %d has H_x, H_y or E_z values: the batch steps TE fields only", i);
   }
   b->reusable = false;
+  drop_places(b);
   auto rebuild = [&](int shape) -> int {
     if (int r = build<T>(b, views, first, parity, rows, shape)) return r;
     if (SHAPES[shape].halo > 0) launch_shape<T>(b, 0, 0, 0);
@@ -1777,6 +1820,7 @@ int run_impl(fdtd_batch *b, int64_t steps, const int64_t *first_steps) {
     b->shape = pick;
   }
   if (int r = rebuild(b->shape)) return r;
+  drop_places(b);
   if (int r = finish_run<T>(b, steps, done, views, &flips)) return r;
   b->reusable = true;
   b->cap_record = b->record;
@@ -1828,13 +1872,15 @@ int solo_run(fdtd_batch *b, bool check, int64_t steps, int64_t first, double *ro
     BTRY(b, cudaMemcpyAsync(&bad, b->d_flags, 4, cudaMemcpyDeviceToHost, b->stream));
     BTRY(b, cudaStreamSynchronize(b->stream));
     if (bad) return 0;
-    if (int r = settle_tm<T>(b, v)) return r;
+    if (int r = settle_tm<T>(b, v, b->d_flags)) return r;
   }
   if (!b->reusable || b->solo_layout != v.layout) {
     b->reusable = false;
     b->aux = v.naux > 0;
     b->shape = block_shape(views, b->sms);
+    drop_places(b);
     if (int r = build<T>(b, views, {first}, {v.parity}, {rows}, b->shape)) return r;
+    drop_places(b);
     launch_shape<T>(b, 0, 0, 0);
     b->solo_layout = v.layout;
     b->reusable = true;
