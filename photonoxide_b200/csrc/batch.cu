@@ -584,11 +584,11 @@ __global__ void te_contract_kernel(const TeInst<T> *insts, const RecItem *items,
   const TeInst<T> &I = insts[it.inst];
   const long long v = it.index;
   const SeriesDev s = I.series[I.value_series[v]];
-  const int f0 = blockIdx.y * DFT_F;
-  if (f0 >= s.nf) return;
-  transform_value<T>(ring + it.col, nring, count, phase + 2 * ((long long)I.slot0 + s.slot0 + f0),
-                     nslots_total, I.sums + 2 * (s.sum0 + (long long)f0 * s.volume + (v - s.value0)),
-                     s.volume, s.nf - f0);
+#pragma unroll 1
+  for (int f0 = blockIdx.y * DFT_F; f0 < s.nf; f0 += gridDim.y * DFT_F)
+    transform_value<T>(ring + it.col, nring, count, phase + 2 * ((long long)I.slot0 + s.slot0 + f0),
+                       nslots_total, I.sums + 2 * (s.sum0 + (long long)f0 * s.volume + (v - s.value0)),
+                       s.volume, s.nf - f0);
 }
 
 // After `count` steps: each instance's step index, current copies (`flips` times the fields',
@@ -963,7 +963,7 @@ struct fdtd_batch {
   int *d_point = nullptr;
   int2 *d_wave_items = nullptr, *d_slot_items = nullptr;
   int nwave_items = 0, nslot_items = 0, nwaves_total = 0, nslots_total = 0;
-  int freq_chunks = 1;  // the most frequencies of a transform, in chunks of DFT_F
+  int freq_chunks = 1;  // rows of the transforms' grid (fdtd_ctx::freq_chunks)
   double *d_waves_h = nullptr, *d_waves_e = nullptr, *d_phase = nullptr;
   RecItem *d_rec = nullptr;
   long long nrec = 0;

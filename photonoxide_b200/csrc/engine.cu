@@ -2303,7 +2303,7 @@ __global__ void phase_kernel(const double *omega, const int *slot_field, int nsl
 __global__ void set_base_kernel(long long *base, long long first) { *base = first; }
 
 // sums[f][v] += sum_m ring[m][v] * phase[m][slot(f)], m in time order, f64 (monitors.rs:185-206):
-// a thread a value and DFT_F of its frequencies (blockIdx.y).
+// a thread a value and DFT_F of its frequencies at a time (blockIdx.y and on by gridDim.y).
 template <typename T>
 __global__ void __launch_bounds__(128) dft_kernel(const SeriesDev *series,
                                                   const long long *value_series, long long nvalues,
@@ -2312,11 +2312,11 @@ __global__ void __launch_bounds__(128) dft_kernel(const SeriesDev *series,
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nvalues) return;
   const SeriesDev s = series[value_series[v]];
-  const int f0 = blockIdx.y * DFT_F;
-  if (f0 >= s.nf) return;
-  transform_value<T>(ring + v, nvalues, batch, phase + 2 * (long long)(s.slot0 + f0), nslots,
-                     sums + 2 * (s.sum0 + (long long)f0 * s.volume + (v - s.value0)), s.volume,
-                     s.nf - f0);
+#pragma unroll 1
+  for (int f0 = blockIdx.y * DFT_F; f0 < s.nf; f0 += gridDim.y * DFT_F)
+    transform_value<T>(ring + v, nvalues, batch, phase + 2 * (long long)(s.slot0 + f0), nslots,
+                       sums + 2 * (s.sum0 + (long long)f0 * s.volume + (v - s.value0)), s.volume,
+                       s.nf - f0);
 }
 
 // The transform of a complex run's values (src/fdtd/monitors.rs:127-154): each step's
@@ -2476,7 +2476,7 @@ struct fdtd_ctx {
   long long *d_where = nullptr, *d_value_series = nullptr;
   SeriesDev *d_series = nullptr;
   int nseries = 0, nslots = 0;
-  int freq_chunks = 1;  // the most frequencies of a series, in chunks of DFT_F
+  int freq_chunks = 1;  // rows of the transforms' grids: the most frequencies of a series in chunks of DFT_F
   double *d_omega = nullptr;
   int *d_slot_field = nullptr;
   long long nsums = 0;
@@ -3944,6 +3944,7 @@ int fdtd_set_dft(fdtd_ctx *c, int32_t nseries, const fdtd_series *series, int32_
   c->sums_taken = 0;
   c->freq_chunks = 1;
   for (const SeriesDev &x : sd) c->freq_chunks = std::max(c->freq_chunks, (x.nf + DFT_F - 1) / DFT_F);
+  c->freq_chunks = std::min(c->freq_chunks, 65535);  // a grid's most rows; the threads go round for the rest
   if (values == 0) return 0;
   // the ring: K steps of the values, K as large as 64 while it stays within 1 GB
   long long K = 64;
