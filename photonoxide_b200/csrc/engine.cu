@@ -3461,7 +3461,10 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
   // 0.228 with 9 or 10, 0.231 with 8, 0.239 with 6 and 0.243 with 13.
   // A run is four planes or more, but where even those leave SMs idle shorter ones, down to one
   // plane: such a grid's step is as long as its longest CTA.
-  const long long slots = (long long)sms * (c->precision == 64 ? quad::ctas<double>() : quad::ctas<float>());
+  // (The other kernels hold more than one CTA an SM in f64 too: cut for one, the row kernel's step of a
+  // 401 x 300 x 40 grid took 556 us and not 489.)
+  const bool one_cta = c->quad && c->precision == 64;
+  const long long slots = (long long)sms * (one_cta ? quad::ctas<double>() : quad::ctas<float>());
   const long long want = 3 * slots;
   int chunks = (int)std::max<long long>(1, (want + tiles - 1) / tiles);
   chunks = std::min(chunks, (int)std::max<long long>(std::max(1, c->n[2] / 4), slots / tiles));
