@@ -2952,6 +2952,9 @@ void launch_aux(fdtd_ctx *c, int stride, long long first, const long long *base,
 bool solo_ok(const fdtd_ctx *c, long long steps) {
   if (c->solo_refused == c->layout || c->forced || c->profiling || c->capturing || steps < SOLO_STEPS || c->te < 0) return false;
   if (c->n[2] != 1 || !c->periodic[2] || c->media || c->nbloch > 0) return false;
+  // a caller that captures the stream: the general kernels' launches are all it can hold
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
   if (c->naux_runs > 0 && !c->aux_te) return false;
   if (c->nvalues > 0 && c->ring_k < 8) return false;  // no ring of a chunk's steps (fdtd_batch::chunk)
   for (const fdtd_injection &x : c->src_inj)

@@ -173,3 +173,35 @@ def test_fields_that_are_not_te_are_looked_at_once(monkeypatch):
     (a1, a2, a), (o1, o2, o) = counts
     assert a1 == o1 + 1 and a2 == o2
     assert np.array_equal(a, o)
+
+
+def test_a_caller_captures_te_steps():
+    """Steps of a TE run enqueued while the caller captures the context's stream: they are captured (on the
+    general kernels, which need no look at the fields and no tables), and replayed they are the same steps."""
+    rt = C.CDLL("libcudart.so.12")
+    out = []
+    for captured in (False, True):
+        s = grid(32)
+        te_fields(s)
+        s.run(2)  # an even number of steps, before and within: a replay finds the same copies current
+        e = Engine(s.engine())
+        stream = C.c_void_p(e.stream())
+        for first in (2, 22):
+            if captured and first == 2:
+                graph, exec_ = C.c_void_p(), C.c_void_p()
+                assert rt.cudaStreamBeginCapture(stream, 1) == 0
+                e.run_async(20, first)
+                assert rt.cudaStreamEndCapture(stream, C.byref(graph)) == 0
+                assert rt.cudaGraphInstantiate(C.byref(exec_), graph, C.c_ulonglong(0)) == 0
+            if captured:
+                assert rt.cudaGraphLaunch(exec_, stream) == 0
+            else:
+                e.run_async(20, first)
+        e.synchronize()
+        if captured:
+            assert rt.cudaGraphExecDestroy(exec_) == 0 and rt.cudaGraphDestroy(graph) == 0
+        n = 3 * s.grid.cells()
+        E, H = np.empty(n), np.empty(n)
+        e.download_fields(E, H)
+        out.append((E, H))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
