@@ -26,7 +26,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <functional>
 #include <mutex>
+#include <queue>
 #include <string>
 #include <memory>
 #include <unordered_map>
@@ -2879,13 +2881,12 @@ int quad_runs(fdtd_ctx *c, int count) {
   return n;
 }
 
-// The quad kernel's CTAs (run r, tile t as r * tiles + t) in launch order: by an estimate of
-// their time, heaviest first, so that the CTAs that start last are short and the step, which
-// ends with its last CTA, leaves few SMs idle at its end. A plane of a tile costs 1, and more
-// where the tile meets a CPML: 0.4 where its rows reach an x CPML, 1.15 times the share of its
-// rows (of 8) in a y CPML, 0.95 in a z CPML's plane; a run's first, recomputed plane of H 0.6 of
-// a plane. (Fitted to the CTAs' times on the 3D MMI, 600 x 200 x 100 with CPMLs of 10.)
-std::vector<int> quad_order(const fdtd_ctx *c) {
+// The quad kernel's CTAs (run r, tile t as r * tiles + t) with an estimate of their time, negated,
+// heaviest first. A plane of a tile costs 1, and more where the tile meets a CPML: 0.4 where its
+// rows reach an x CPML, 1.15 times the share of its rows (of 8) in a y CPML, 0.95 in a z CPML's
+// plane; a run's first, recomputed plane of H 0.6 of a plane. (Fitted to the CTAs' times on the 3D
+// MMI, 600 x 200 x 100 with CPMLs of 10.)
+std::vector<std::pair<double, int>> quad_costs(const fdtd_ctx *c) {
   const int nx = c->n[0], ny = c->n[1], nz = c->n[2];
   const int tiles = c->tiles_x * c->tiles_y;
   auto zslab = [&](int k) { return !c->periodic[2] && (k < c->low[2] || k >= nz - c->high[2]); };
@@ -2912,9 +2913,32 @@ std::vector<int> quad_order(const fdtd_ctx *c) {
                    [](const std::pair<double, int> &a, const std::pair<double, int> &b) {
                      return a.first < b.first;
                    });
+  return cost;
+}
+
+// Their launch order: heaviest first, so that the CTAs that start last are short and the step, which
+// ends with its last CTA, leaves few SMs idle at its end.
+std::vector<int> quad_order(const fdtd_ctx *c) {
+  const std::vector<std::pair<double, int>> cost = quad_costs(c);
   std::vector<int> order(cost.size());
   for (size_t i = 0; i < cost.size(); i++) order[i] = cost[i].second;
   return order;
+}
+
+// When the last CTA ends, by that estimate, where the device holds `slots` CTAs at a time.
+double quad_span(const fdtd_ctx *c, long long slots) {
+  std::priority_queue<double, std::vector<double>, std::greater<double>> ends;
+  double span = 0.0;
+  for (const auto &q : quad_costs(c)) {
+    double at = 0.0;
+    if ((long long)ends.size() >= slots) {
+      at = ends.top();
+      ends.pop();
+    }
+    ends.push(at - q.first);
+    span = std::max(span, at - q.first);
+  }
+  return span;
 }
 
 // The rows of a tile that the source tables tell apart: the quad kernel's, a warp each.
@@ -3477,10 +3501,17 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
   c->zchunk = (c->n[2] + chunks - 1) / chunks;
   c->zchunks = (c->n[2] + c->zchunk - 1) / c->zchunk;
   if (c->quad) {
-    c->zchunks = quad_runs(c, chunks);
-    // short runs: no more CTAs than the device holds at once (the CPMLs' runs come on top)
-    if (c->n[2] / 4 < slots / tiles)
+    // short runs: no more CTAs than the device holds at once (the CPMLs' runs come on top), unless runs of
+    // four planes and more, a few CTAs beyond that, are estimated to end sooner (a 124 x 300 x 20 grid with
+    // CPMLs of 6: 301 CTAs of up to 3 planes take 32 us a step, 172 of up to 6 took 54)
+    const int plain = std::min(chunks, std::max(1, c->n[2] / 4));
+    c->zchunks = quad_runs(c, zc ? chunks : plain);
+    if (!zc && chunks > plain) {
+      const double span = quad_span(c, slots);
+      c->zchunks = quad_runs(c, chunks);
       for (int q = chunks - 1; q > 1 && c->zchunks * tiles > slots; q--) c->zchunks = quad_runs(c, q);
+      if (quad_span(c, slots) >= span) c->zchunks = quad_runs(c, plain);
+    }
     const std::vector<int> order = quad_order(c);
     if (int r = alloc(c, (void **)&c->order, order.size() * 4)) return r;
     CUDA_TRY(c, copy(c, c->order, order.data(), order.size() * 4, cudaMemcpyHostToDevice));
