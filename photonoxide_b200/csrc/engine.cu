@@ -797,11 +797,49 @@ __device__ __forceinline__ SlabEntry zslab_of(const StepArgs<T> &A, int field, i
   return none;
 }
 
+// The sources of one field at a warp's row and plane of the row kernel: the groups g0 .. g1-1, a lane a
+// group, through `rows`, the warp's own three rows of SEG (the quad kernel's inject_row, for two places a
+// lane). cb: E's coefficients from the row's first value on; x: where the row's place 0 is along it.
+template <typename T, int FIELD>
+__device__ __forceinline__ void inject_places(const StepArgs<T> &A, int g0, int g1, T *rows, const T *cb, int x,
+                                              int lane, T v[3][2]) {
+  if (g1 <= g0) return;
+  using rowstep::SEG;
+  const Group *groups = FIELD == 1 ? A.hgroups : A.egroups;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    rows[c * SEG + lane] = v[c][0];
+    rows[c * SEG + lane + 32] = v[c][1];
+  }
+  __syncwarp();
+  for (int g = g0 + lane; g < g1; g += 32) {
+    const Group gr = groups[g];
+    const int pos = gr.local % SEG;
+    T *at = rows + gr.comp * SEG + pos;
+    T u = *at;
+    if (FIELD == 1) {
+      for (int q = gr.first; q < gr.first + gr.count; q++) u = apply_h<T>(u, A.entries[q], A.waves_h, A.dt);
+    } else {
+      const T cbv = cb[gr.comp * A.N + x + pos];  // an owned place: in the grid's row
+      for (int q = gr.first; q < gr.first + gr.count; q++) u = apply_e<T>(u, A.entries[q], A.waves_e, cbv);
+    }
+    *at = u;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    v[c][0] = rows[c * SEG + lane];
+    v[c][1] = rows[c * SEG + lane + 32];
+  }
+  __syncwarp();  // (the rows are written again at the next sources)
+}
+
 template <typename T, bool LOSSY, bool MEDIA>
 __global__ void __launch_bounds__(rowstep::THREADS, 2) row_kernel(StepArgs<T> A) {
   using namespace rowstep;
   __shared__ T sE[2][WARPS][SEG];  // E_x, E_z of plane k, each warp's row (for the row above)
   __shared__ T sH[2][WARPS][SEG];  // H_x, H_z of plane k (for the row below)
+  __shared__ T sS[WARPS][3 * SEG];  // a row's values while its sources are added
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nx = A.n[0], ny = A.n[1], nz = A.n[2];
   const long long N = A.N;
@@ -809,7 +847,10 @@ __global__ void __launch_bounds__(rowstep::THREADS, 2) row_kernel(StepArgs<T> A)
   const int x0 = (tile % A.tiles_x) * OWN, y0 = (tile / A.tiles_x) * RW;
   const int kbeg = blockIdx.y * A.zchunk, kend = min(kbeg + A.zchunk, nz);
   if (kbeg >= nz) return;
-  const int tileidx = tile;
+  // whether the tile has currents in any plane (most have none: then no plane looks them up)
+  const long long tile_rows = (long long)tile * nz * WARPS;
+  const bool hcur = A.hbucket[tile_rows] != A.hbucket[tile_rows + (long long)nz * WARPS];
+  const bool ecur = A.ebucket[tile_rows] != A.ebucket[tile_rows + (long long)nz * WARPS];
 
   // -- per lane: the two x places; per warp: the row
   int gx[2], mx[2], mxp[2];
@@ -966,28 +1007,10 @@ __global__ void __launch_bounds__(rowstep::THREADS, 2) row_kernel(StepArgs<T> A)
       hn[1][h] = hy;
       hn[2][h] = hz;
     }
-    // the magnetic currents at this tile and plane, each value's entries in CPU order
-    const int bucket = tileidx * nz + k;
-    const int g0 = A.hbucket[bucket], g1 = A.hbucket[bucket + 1];
-    for (int g = g0; g < g1; g++) {
-      Group gr = A.hgroups[g];
-      int gw = gr.local / SEG, gi = gr.local % SEG;
-      if (gw == w && (gi & 31) == lane) {
-        const bool second = (gi >> 5) != 0;
-        T v = T(0);
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-          if (gr.comp == c) v = second ? hn[c][1] : hn[c][0];
-        for (int q = gr.first; q < gr.first + gr.count; q++) {
-          v = apply_h<T>(v, A.entries[q], A.waves_h, A.dt);
-        }
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-          if (gr.comp == c) {
-            if (second) hn[c][1] = v;
-            else hn[c][0] = v;
-          }
-      }
+    // the magnetic currents of the row, each value's entries in CPU order
+    if (hcur) {
+      const long long bucket = tile_rows + k * WARPS + w;
+      inject_places<T, 1>(A, A.hbucket[bucket], A.hbucket[bucket + 1], sS[w], nullptr, 0, lane, hn);
     }
   };
 
@@ -1089,32 +1112,9 @@ __global__ void __launch_bounds__(rowstep::THREADS, 2) row_kernel(StepArgs<T> A)
       hprev[1][h] = hn[1][h];
     }
     // the electric currents (src/fdtd.rs:1375-1387)
-    {
-      const int bucket = tileidx * nz + k;
-      const int g0 = A.ebucket[bucket], g1 = A.ebucket[bucket + 1];
-      for (int g = g0; g < g1; g++) {
-        Group gr = A.egroups[g];
-        int gw = gr.local / SEG, gi = gr.local % SEG;
-        if (gw == w && (gi & 31) == lane) {
-          const bool second = (gi >> 5) != 0;
-          T cbv = T(0), v = T(0);
-#pragma unroll
-          for (int c = 0; c < 3; c++)
-            if (gr.comp == c) {
-              cbv = second ? P.cb[c][1] : P.cb[c][0];
-              v = second ? en[c][1] : en[c][0];
-            }
-          for (int q = gr.first; q < gr.first + gr.count; q++) {
-            v = apply_e<T>(v, A.entries[q], A.waves_e, cbv);
-          }
-#pragma unroll
-          for (int c = 0; c < 3; c++)
-            if (gr.comp == c) {
-              if (second) en[c][1] = v;
-              else en[c][0] = v;
-            }
-        }
-      }
+    if (ecur) {
+      const long long bucket = tile_rows + k * WARPS + w;
+      inject_places<T, 0>(A, A.ebucket[bucket], A.ebucket[bucket + 1], sS[w], A.cb + pk + rowoff, x0 - 1, lane, en);
     }
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -1166,7 +1166,7 @@ __global__ void __launch_bounds__(rowstep::THREADS, 2) row_kernel(StepArgs<T> A)
 
 
 // ------------------------------------------------------------------------------------------
-// The quad step (v3), the default where nx is a multiple of 4. A CTA owns OWNX = 124 values along
+// The quad step (v3), the default (row_better: but for some narrow grids). A CTA owns OWNX = 124 values along
 // x and RW rows along y of a run of planes. Warp w holds row y0 - 1 + w; lane l holds the four
 // values x0 - 4 + 4l .. x0 - 1 + 4l of it (128 a row: the tile's 124 and the 4 before it, whose
 // last H the tile's first E needs). Every global access is a 16-byte vector. The next plane's E,
@@ -2941,8 +2941,8 @@ double quad_span(const fdtd_ctx *c, long long slots) {
   return span;
 }
 
-// The rows of a tile that the source tables tell apart: the quad kernel's, a warp each.
-int bucket_rows(const fdtd_ctx *c) { return c->quad ? quad::WARPS : 1; }
+// The rows of a tile that the source tables tell apart: the quad and the row kernel's, a warp each.
+int bucket_rows(const fdtd_ctx *c) { return c->quad ? quad::WARPS : c->row ? rowstep::WARPS : 1; }
 
 // Empty source tables: every bucket empty.
 int empty_sources(fdtd_ctx *c) {
@@ -3281,6 +3281,30 @@ int bloch_impl(fdtd_ctx *a, fdtd_ctx *b, const std::vector<WrapDev> &hw,
   return 0;
 }
 
+// Whether the row kernel steps a 3D grid of rows that are no whole vectors, between walls or CPMLs, faster than
+// the quad kernel's value-by-value form. A row of either costs much the same however many of its places the
+// grid has, and the row kernel's is 63 places (two passes of 32 lanes, the second skipped where it has none),
+// the quad kernel's 124: so on narrow grids, and on those just past 124, the row kernel has no more columns of
+// tiles, each cheaper. A CPML along y or z costs it more than the quad kernel, which takes four places of a row
+// of psi at once; a CPML along x on both ends of the same row costs the quad kernel more; and in f64 the quad
+// kernel has one CTA an SM, a long step where the CTAs are few. us a step, row and quad, 1128 grids timed: f32
+// walls 61 x 150 x 100 27 and 37, 187 x 150 x 100 84 and 79; x CPMLs alone 51 x 33 x 250 35 and 54; all CPMLs 21 x 33 x 250 40 and 55, 33 x 150 x 100
+// 84 and 68, 61 x 60 x 60 34 and 24; f64 all CPMLs 25 x 150 x 100 87 and 145, 33 x 33 x 250 96 and 102, 61 x 150
+// x 100 174 and 166, 61 x 60 x 60 47 and 78, 99 x 60 x 60 75 and 69. (One cell thick, the quad kernel needs no
+// plane before the first: 33 x 17 11 and 13.)
+bool row_better(const fdtd_ctx *c) {
+  const int nx = c->n[0];
+  if (nx % 4 == 0 || c->n[2] == 1) return false;
+  if (nx <= 31) return true;
+  const int rows = (nx + rowstep::OWN - 1) / rowstep::OWN, quads = (nx + quad::OWNX - 1) / quad::OWNX;
+  const bool f64 = c->precision == 64;
+  const bool yz = c->low[1] + c->high[1] + c->low[2] + c->high[2] > 0;
+  if (rows != quads) return false;
+  if (!yz) return true;
+  const long long ctas = (long long)quads * ((c->n[1] + quad::RW - 1) / quad::RW) * std::max(1, c->n[2] / 4);
+  return f64 && (ctas <= c->sms || (nx <= 37 && c->low[0] + c->high[0] > 0));
+}
+
 }  // namespace
 
 extern "C" {
@@ -3361,7 +3385,6 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
     N *= c->n[a];
   }
   c->N = N;
-  c->pitch = (c->n[0] + 3) / 4 * 4;
   *out = c;
   if (!(dt > 0.0 && std::isfinite(dt)))
     return fail(c, FDTD_E_INVALID, "the time step must be positive, got %g", dt);
@@ -3377,6 +3400,29 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
   if (int r = alloc(c, &c->fh, nf * E)) return r;
   if (int r = upload(c, c->fe, factor_e, nf)) return r;
   if (int r = upload(c, c->fh, factor_h, nf)) return r;
+  {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  {
+    const char *force = getenv("PHOTONOXIDE_FDTD_KERNEL");
+    // the quad kernel takes four places along x at once: nx a multiple of 4 or ends along x that
+    // don't wrap (a wrapped group of four would straddle two rows' ends), and no group of four
+    // holding places of both x CPMLs (an interior narrower than the group); its offsets within a
+    // plane are ints
+    const bool quad_ok = (c->n[0] % 4 == 0 || !c->periodic[0]) &&
+        !(c->low[0] > 0 && c->high[0] > 0 && (c->low[0] - 1) / 4 == (c->n[0] - c->high[0]) / 4) &&
+        (long long)c->n[0] * c->n[1] < (1LL << 31);
+    std::string kind = force ? force : (quad_ok && !row_better(c) ? "quad" : "row");
+    if (kind == "quad" && !quad_ok) kind = "row";
+    c->forced = force != nullptr;
+    c->quad = kind == "quad";
+    c->row = kind == "row";
+    c->staged = kind == "staged" && (c->n[0] % (16 / (int)c->elem) == 0);
+  }
+  // the quad kernel takes psi's rows four places at a time: whole vectors (padding costs the others bytes)
+  c->pitch = c->quad ? (c->n[0] + 3) / 4 * 4 : c->n[0];
   // the slabs: psi for E in place, for H in two copies; their coefficients in one table
   memset(c->table, 0, sizeof c->table);
   std::vector<double> coefs;
@@ -3432,13 +3478,7 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
   // several CTAs per SM
   c->tiles_x = (c->n[0] + TX - 1) / TX;
   c->tiles_y = (c->n[1] + TY - 1) / TY;
-  int sms = 148;
-  {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  }
-  c->sms = sms;
+  const int sms = c->sms;
   // the slabs' d/h: in f32 by the product form where it is checked to give division's bits
   for (int a = 0; a < 3; a++) {
     if (c->precision == 64) {
@@ -3449,22 +3489,6 @@ int fdtd_create(const fdtd_grid *grid, double dt, const double step[3], const do
     const float h = (float)c->step[a], r = (float)(1.0 / (double)h);
     c->inv_step[a] = r;
     if (int q = division_checked(c, h, r, &c->fast_div[a])) return q;
-  }
-  {
-    const char *force = getenv("PHOTONOXIDE_FDTD_KERNEL");
-    // the quad kernel takes four places along x at once: nx a multiple of 4 or ends along x that
-    // don't wrap (a wrapped group of four would straddle two rows' ends), and no group of four
-    // holding places of both x CPMLs (an interior narrower than the group); its offsets within a
-    // plane are ints
-    const bool quad_ok = (c->n[0] % 4 == 0 || !c->periodic[0]) &&
-        !(c->low[0] > 0 && c->high[0] > 0 && (c->low[0] - 1) / 4 == (c->n[0] - c->high[0]) / 4) &&
-        (long long)c->n[0] * c->n[1] < (1LL << 31);
-    std::string kind = force ? force : (quad_ok ? "quad" : "row");
-    if (kind == "quad" && !quad_ok) kind = "row";
-    c->forced = force != nullptr;
-    c->quad = kind == "quad";
-    c->row = kind == "row";
-    c->staged = kind == "staged" && (c->n[0] % (16 / (int)c->elem) == 0);
   }
   if (c->row) {
     c->tile_w = rowstep::OWN;

@@ -32,7 +32,8 @@ def fields(s):
 
 
 W, L = Pml(0, 0), Pml(3, 4)
-CASES = [((7, 9, 5), (W, W, W)), ((33, 9, 6), (L, L, W)), ((123, 8, 9), (L, Periodic(), L)),
+CASES = [((1, 9, 5), (W, L, W)), ((2, 9, 12), (Pml(0, 1), W, L)), ((3, 17, 5), (Pml(1, 0), Periodic(), W)),
+         ((3, 9, 5), (W, W, W)), ((7, 9, 5), (W, W, W)), ((33, 9, 6), (L, L, W)), ((123, 8, 9), (L, Periodic(), L)),
          ((125, 15, 4), (L, W, Periodic())), ((126, 8, 9), (W, L, L)), ((249, 14, 3), (L, L, Periodic())),
          ((45, 30, 1), (Pml(20, 17), L, Periodic())), ((37, 21, 19), (L, L, L))]
 
@@ -41,17 +42,20 @@ CASES = [((7, 9, 5), (W, W, W)), ((33, 9, 6), (L, L, W)), ((123, 8, 9), (L, Peri
 @pytest.mark.parametrize("lossy,media", [(False, False), (True, False), (True, True)])
 def test_ragged_rows(monkeypatch, n, edges, lossy, media):
     from pyoracle import OracleSimulation
+    d = stirred(lambda *q: Simulation(*q, precision=64), n, edges, lossy, media)  # the kernel it gets
+    d.run(12)
+    monkeypatch.setenv("PHOTONOXIDE_FDTD_KERNEL", "quad")
     a = stirred(lambda *q: Simulation(*q, precision=64), n, edges, lossy, media)
     o = stirred(lambda *q: OracleSimulation(*q, precision=64), n, edges, lossy, media)
     f = stirred(lambda *q: Simulation(*q, precision=32), n, edges, lossy, media)
     f.run(12)
+    a.run(12)
     monkeypatch.setenv("PHOTONOXIDE_FDTD_KERNEL", "row")
     g = stirred(lambda *q: Simulation(*q, precision=32), n, edges, lossy, media)
     g.run(12)
-    for s in (a, o):
-        s.run(12)
-    for x, y in zip(fields(a), fields(o)):
-        assert np.array_equal(x, y)
+    o.run(12)
+    for x, y, z in zip(fields(a), fields(o), fields(d)):
+        assert np.array_equal(x, y) and np.array_equal(z, y)
     for x, y in zip(fields(f), fields(g)):
         assert np.array_equal(x, y)
 

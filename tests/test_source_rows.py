@@ -1,6 +1,6 @@
 """Many sources on a row: currents over whole rows and tile edges, two on the same values, as a
-plane wave's box or a Bloch side gives them. The quad kernel takes a row's values a lane each, more
-than 32 in turn; in f64 every value is the oracle's bits, in f32 within the reference's GPU tolerance
+plane wave's box or a Bloch side gives them. The quad kernel, and the row kernel (rows that are no whole
+vectors, narrow or wrapped), take a row's values a lane each, more than 32 in turn; in f64 every value is the oracle's bits, in f32 within the reference's GPU tolerance
 (2e-5 of the largest value, src/fdtd/gpu/tests.rs:51-66)."""
 import numpy as np
 import pytest
@@ -29,7 +29,7 @@ def problem(make, n, periodic, lossy):
     return s
 
 
-@pytest.mark.parametrize("n", [(4, 8, 5), (128, 15, 6), (252, 9, 5)])
+@pytest.mark.parametrize("n", [(4, 8, 5), (128, 15, 6), (252, 9, 5), (27, 15, 6), (131, 9, 5)])
 @pytest.mark.parametrize("periodic", [False, True])
 @pytest.mark.parametrize("precision,lossy", [(64, False), (64, True), (32, False), (32, True)])
 def test_rows_of_sources_match_the_oracle(n, periodic, precision, lossy):
