@@ -204,9 +204,12 @@ int fdtd_set_media(fdtd_ctx *ctx, int32_t ngroups, const fdtd_media_group *group
  * sources' and transforms' times), as Resident::step (resident.rs:430-539). Returns when the
  * device is done. */
 int fdtd_run(fdtd_ctx *ctx, int64_t steps, int64_t first_step);
-/* The same, enqueued on the context's stream without waiting (for timing and overlap). A 2D run of TE
- * sources whose fields have come from elsewhere since its last run (uploaded, or handed out by
- * fdtd_device_fields) first waits for the context's earlier work, to see whether they are TE. */
+/* The same, enqueued on the context's stream without waiting (for timing and overlap). A 2D run of 16
+ * steps or more whose sources are TE does more before it returns, unless the stream is being captured: after
+ * the fields have come from elsewhere (uploaded, or handed out by fdtd_device_fields) it waits for the
+ * context's earlier work, to see whether they are TE, and after the coefficients, sources, probes or
+ * transforms were set it makes its tables on the host and allocates them (from the HBM budget; without room
+ * for them the general kernels step). */
 int fdtd_run_async(fdtd_ctx *ctx, int64_t steps, int64_t first_step);
 int fdtd_synchronize(fdtd_ctx *ctx);
 
@@ -226,7 +229,9 @@ void *fdtd_stream(fdtd_ctx *ctx);
 /* The kernels the last run launched, for accounting. */
 int64_t fdtd_launches(const fdtd_ctx *ctx);
 /* With `on`, each launch of the step kernel is bracketed by CUDA events on the context's stream;
- * fdtd_profile_read gives their summed device time (ms) and count since profiling started. */
+ * fdtd_profile_read gives their summed device time (ms) and count since profiling started. Every run then
+ * takes the general kernels, a step a launch: of a 2D TE run, which otherwise takes several steps a launch on
+ * tiles of its own, the time is those kernels'. */
 int fdtd_profile(fdtd_ctx *ctx, int32_t on);
 int fdtd_profile_read(fdtd_ctx *ctx, double *ms, int64_t *launches);
 

@@ -2335,7 +2335,7 @@ int fdtd_adjoint_create(fdtd_ctx *ctx, int64_t steps, int32_t segment, int64_t c
   if (count <= 0 || !component || !r) return afail(a, FDTD_E_INVALID, "a design needs values");
   a->ctx = ctx;
   a->steps = steps;
-  a->segment = segment + (segment & 1);  // even: every checkpoint has the same current copy
+  a->segment = segment + (segment & 1);
   a->nseg = (int)((steps + a->segment - 1) / a->segment);
   InstanceView v;
   if (int q = fdtd_instance_view(ctx, &v)) return afail(a, q, "%s", fdtd_last_error(ctx));
