@@ -576,7 +576,7 @@ __global__ void te_record_kernel(const TeInst<T> *insts, const RecItem *items, l
 template <typename T>
 __global__ void te_contract_kernel(const TeInst<T> *insts, const RecItem *items, long long nitems,
                                    const T *ring, long long nring, const double *phase,
-                                   int nslots_total, int count) {
+                                   int nslots_total, int count, int row0) {
   long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nitems) return;
   const RecItem it = items[q];
@@ -584,11 +584,11 @@ __global__ void te_contract_kernel(const TeInst<T> *insts, const RecItem *items,
   const TeInst<T> &I = insts[it.inst];
   const long long v = it.index;
   const SeriesDev s = I.series[I.value_series[v]];
-#pragma unroll 1
-  for (int f0 = blockIdx.y * DFT_F; f0 < s.nf; f0 += gridDim.y * DFT_F)
-    transform_value<T>(ring + it.col, nring, count, phase + 2 * ((long long)I.slot0 + s.slot0 + f0),
-                       nslots_total, I.sums + 2 * (s.sum0 + (long long)f0 * s.volume + (v - s.value0)),
-                       s.volume, s.nf - f0);
+  const int f0 = (row0 + blockIdx.y) * DFT_F;
+  if (f0 >= s.nf) return;
+  transform_value<T>(ring + it.col, nring, count, phase + 2 * ((long long)I.slot0 + s.slot0 + f0),
+                     nslots_total, I.sums + 2 * (s.sum0 + (long long)f0 * s.volume + (v - s.value0)),
+                     s.volume, s.nf - f0);
 }
 
 // After `count` steps: each instance's step index, current copies (`flips` times the fields',
@@ -963,7 +963,7 @@ struct fdtd_batch {
   int *d_point = nullptr;
   int2 *d_wave_items = nullptr, *d_slot_items = nullptr;
   int nwave_items = 0, nslot_items = 0, nwaves_total = 0, nslots_total = 0;
-  int freq_chunks = 1;  // rows of the transforms' grid (fdtd_ctx::freq_chunks)
+  int freq_chunks = 1;  // the most frequencies of a transform, in chunks of DFT_F
   double *d_waves_h = nullptr, *d_waves_e = nullptr, *d_phase = nullptr;
   RecItem *d_rec = nullptr;
   long long nrec = 0;
@@ -1543,11 +1543,10 @@ int enqueue(fdtd_batch *b, int count) {
       b->launches++;
     }
   }
-  if (b->nring > 0 && b->record) {
-    te_contract_kernel<T><<<dim3((unsigned)((b->nrec + 127) / 128), b->freq_chunks), 128, 0,
-                            b->stream>>>(
-        insts, b->d_rec, b->nrec, (const T *)b->d_ring, b->nring, b->d_phase, b->nslots_total,
-        count);
+  for (int row = 0; b->nring > 0 && b->record && row < b->freq_chunks; row += DFT_ROWS) {
+    const dim3 grid((unsigned)((b->nrec + 127) / 128), std::min(DFT_ROWS, b->freq_chunks - row));
+    te_contract_kernel<T><<<grid, 128, 0, b->stream>>>(insts, b->d_rec, b->nrec, (const T *)b->d_ring,
+                                                       b->nring, b->d_phase, b->nslots_total, count, row);
     b->launches++;
   }
   te_advance_kernel<T><<<(n + 127) / 128, 128, 0, b->stream>>>(insts, n, count, flips, psi_flips);

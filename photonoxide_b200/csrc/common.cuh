@@ -153,6 +153,7 @@ __device__ __forceinline__ void transform_chunk(const T *ring, long long row, in
 // plane's six components at 21 frequencies, 64 steps a batch, took 353 us with one frequency after
 // another in each thread, and the 25 196 flux values of the 3D splitter at 51 frequencies 127 us.
 constexpr int DFT_F = 8;
+constexpr int DFT_ROWS = 65535;  // the chunks of DFT_F a launch's rows can be
 template <typename T>
 __device__ __forceinline__ void transform_value(const T *ring, long long row, int batch,
                                                 const double *ph, int slots, double *acc,

@@ -2305,20 +2305,21 @@ __global__ void phase_kernel(const double *omega, const int *slot_field, int nsl
 __global__ void set_base_kernel(long long *base, long long first) { *base = first; }
 
 // sums[f][v] += sum_m ring[m][v] * phase[m][slot(f)], m in time order, f64 (monitors.rs:185-206):
-// a thread a value and DFT_F of its frequencies at a time (blockIdx.y and on by gridDim.y).
+// a thread a value and DFT_F of its frequencies (row0 + blockIdx.y). A launch has 65 535 rows, so more
+// frequencies are more launches: a loop over them in the kernel cost a run with whole-plane transforms 2 %.
 template <typename T>
 __global__ void __launch_bounds__(128) dft_kernel(const SeriesDev *series,
                                                   const long long *value_series, long long nvalues,
                                                   const T *ring, int batch, const double *phase,
-                                                  int nslots, double *sums) {
+                                                  int nslots, double *sums, int row0) {
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nvalues) return;
   const SeriesDev s = series[value_series[v]];
-#pragma unroll 1
-  for (int f0 = blockIdx.y * DFT_F; f0 < s.nf; f0 += gridDim.y * DFT_F)
-    transform_value<T>(ring + v, nvalues, batch, phase + 2 * (long long)(s.slot0 + f0), nslots,
-                       sums + 2 * (s.sum0 + (long long)f0 * s.volume + (v - s.value0)), s.volume,
-                       s.nf - f0);
+  const int f0 = (row0 + blockIdx.y) * DFT_F;
+  if (f0 >= s.nf) return;
+  transform_value<T>(ring + v, nvalues, batch, phase + 2 * (long long)(s.slot0 + f0), nslots,
+                     sums + 2 * (s.sum0 + (long long)f0 * s.volume + (v - s.value0)), s.volume,
+                     s.nf - f0);
 }
 
 // The transform of a complex run's values (src/fdtd/monitors.rs:127-154): each step's
@@ -2478,7 +2479,7 @@ struct fdtd_ctx {
   long long *d_where = nullptr, *d_value_series = nullptr;
   SeriesDev *d_series = nullptr;
   int nseries = 0, nslots = 0;
-  int freq_chunks = 1;  // rows of the transforms' grids: the most frequencies of a series in chunks of DFT_F
+  int freq_chunks = 1;  // the most frequencies of a series, in chunks of DFT_F
   double *d_omega = nullptr;
   int *d_slot_field = nullptr;
   long long nsums = 0;
@@ -3084,10 +3085,14 @@ int run_impl(fdtd_ctx *c, long long steps, long long first) {
       phase_kernel<<<(total + 127) / 128, 128, 0, c->stream>>>(c->d_omega, c->d_slot_field,
                                                                 c->nslots, first + at, base,
                                                                 batch, c->dt, c->phase);
-      dft_kernel<T><<<dim3((unsigned)((c->nvalues + 127) / 128), c->freq_chunks), 128, 0,
-                      c->stream>>>(c->d_series, c->d_value_series, c->nvalues, (const T *)c->ring,
-                                   batch, c->phase, c->nslots, c->sums);
-      c->launches += 2;
+      c->launches++;
+      for (int row = 0; row < c->freq_chunks; row += DFT_ROWS) {
+        const dim3 grid((unsigned)((c->nvalues + 127) / 128), std::min(DFT_ROWS, c->freq_chunks - row));
+        dft_kernel<T><<<grid, 128, 0, c->stream>>>(c->d_series, c->d_value_series, c->nvalues,
+                                                   (const T *)c->ring, batch, c->phase, c->nslots,
+                                                   c->sums, row);
+        c->launches++;
+      }
     }
   };
   // whole batches replay a captured graph (K even: a batch leaves the current copy as it found
@@ -4009,7 +4014,6 @@ int fdtd_set_dft(fdtd_ctx *c, int32_t nseries, const fdtd_series *series, int32_
   c->sums_taken = 0;
   c->freq_chunks = 1;
   for (const SeriesDev &x : sd) c->freq_chunks = std::max(c->freq_chunks, (x.nf + DFT_F - 1) / DFT_F);
-  c->freq_chunks = std::min(c->freq_chunks, 65535);  // a grid's most rows; the threads go round for the rest
   if (values == 0) return 0;
   // the ring: K steps of the values, K as large as 64 while it stays within 1 GB
   long long K = 64;

@@ -36,8 +36,7 @@ struct InstanceView {
   long long nsums;  // complex sums
   void *ring;  // the transforms' ring: ring_k rows of nvalues
   int ring_k;
-  int freq_chunks;  // rows of the transforms' grids: the most frequencies of a series in chunks of DFT_F
-                    // (at least 1, at most 65535)
+  int freq_chunks;  // the most frequencies of a series, in chunks of DFT_F (at least 1)
   int nprobes;
   const long long *probes;
   bool media;
