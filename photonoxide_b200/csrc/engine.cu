@@ -4173,6 +4173,10 @@ int fdtd_read_dft(fdtd_ctx *c, double *sums, int64_t count) {
     return fail(c, FDTD_E_INVALID, "the transforms hold %lld sums, not %lld", c->nsums, (long long)count);
   if (c->nsums == 0) return 0;
   const long long n = 2 * c->nsums;
+  if (c->sums_taken) {  // what an earlier read took and could not clear
+    CUDA_TRY(c, cudaMemsetAsync(c->sums, 0, c->sums_taken * 8, c->stream));
+    c->sums_taken = 0;
+  }
   if (void *dev = mapped_range(sums, (size_t)n * 8)) {
     // added over the link into the caller's mapped array
     add_into_kernel<<<stride_blocks(c, n), 256, 0, c->stream>>>(c->sums, (double *)dev, n);
