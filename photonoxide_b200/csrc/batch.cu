@@ -1072,6 +1072,23 @@ int zeros(fdtd_batch *b, double **dst, size_t n) {
   return 0;
 }
 
+// Along one axis of n places (wrapping where periodic): the tiles of `own` places whose regions of `len`, from
+// `halo` before a tile's first place on, hold place c, and where in the region; every wrapped image.
+std::vector<std::pair<int, int>> region_images(int c, int n, int own, int halo, int len, int tiles, int periodic) {
+  std::vector<std::pair<int, int>> out;
+  for (int t = 0; t < tiles; t++) {
+    const int lo = t * own - halo;
+    if (!periodic) {
+      if (c >= lo && c < lo + len) out.push_back({t, c - lo});
+      continue;
+    }
+    int first = (c - lo) % n;
+    if (first < 0) first += n;
+    for (int q = first; q < len; q += n) out.push_back({t, q});
+  }
+  return out;
+}
+
 int read_places(fdtd_batch *b, const std::vector<InstanceView> &views) {
   const size_t n = views.size();
   b->where.assign(n, {});
@@ -1238,23 +1255,8 @@ int build(fdtd_batch *b, const std::vector<InstanceView> &views, const std::vect
           to.push_back(c);
         };
         if (halo > 0) {
-          // every place of every region that holds the value, wrapped images included
-          std::vector<std::pair<int, int>> px, py;
-          auto images = [&](int c, int n, int w, int len, int tiles, int periodic,
-                            std::vector<std::pair<int, int>> &out) {
-            for (int t = 0; t < tiles; t++) {
-              const int lo = t * w - halo;  // the region's first place
-              if (!periodic) {
-                if (c >= lo && c < lo + len) out.push_back({t, c - lo});
-                continue;
-              }
-              int first = (c - lo) % n;
-              if (first < 0) first += n;
-              for (int q = first; q < len; q += n) out.push_back({t, q});
-            }
-          };
-          images(x, I.nx, TW, BW, I.tiles_x, I.px, px);
-          images(y, I.ny, TH, bh, tiles_y, I.py, py);
+          const auto px = region_images(x, I.nx, TW, halo, BW, I.tiles_x, I.px);
+          const auto py = region_images(y, I.ny, TH, halo, bh, tiles_y, I.py);
           for (auto oy : py)
             for (auto ox : px)
               add((f ? hper : eper)[oy.first * I.tiles_x + ox.first], oy.second * BW + ox.second);
@@ -2150,28 +2152,13 @@ int adjoint_tables(fdtd_adjoint *a, const InstanceView &v, const std::vector<lon
   a->tiles_x = (nx + TW - 1) / TW;
   const int tiles_y = (ny + TH - 1) / TH;
   a->tiles = a->tiles_x * tiles_y;
-  // the places of every region that hold a value, wrapped images included (build)
-  auto images = [&](int c, int n, int w, int len, int tiles, int periodic) {
-    std::vector<std::pair<int, int>> out;
-    for (int t = 0; t < tiles; t++) {
-      const int lo = t * w - halo;
-      if (!periodic) {
-        if (c >= lo && c < lo + len) out.push_back({t, c - lo});
-        continue;
-      }
-      int first = (c - lo) % n;
-      if (first < 0) first += n;
-      for (int q = first; q < len; q += n) out.push_back({t, q});
-    }
-    return out;
-  };
   std::vector<std::vector<AdjOwner>> eo(a->tiles), ho(a->tiles);
   for (size_t g = 0; g < owner.size(); g++) {
     const bool hf = (owner[g] >> 62) != 0;
     const long long place = owner[g] & ((1LL << 62) - 1), r = place % v.N;
     const int comp = hf ? 2 : (int)(place / v.N);
-    for (auto oy : images((int)(r / nx), ny, TH, TH + 2 * halo, tiles_y, v.periodic[1]))
-      for (auto ox : images((int)(r % nx), nx, TW, BW, a->tiles_x, v.periodic[0]))
+    for (auto oy : region_images((int)(r / nx), ny, TH, halo, TH + 2 * halo, tiles_y, v.periodic[1]))
+      for (auto ox : region_images((int)(r % nx), nx, TW, halo, BW, a->tiles_x, v.periodic[0]))
         (hf ? ho : eo)[oy.first * a->tiles_x + ox.first].push_back(
             AdjOwner{oy.second * BW + ox.second, comp, start[g], start[g + 1] - start[g]});
   }
