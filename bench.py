@@ -531,8 +531,8 @@ def _te_instances(count, seed=0, precision=32):
 def workload_batch(args):
     """Configuration 4, forward: 64 uneven 2D TE instances (sides log-uniform 256-1024 cells) with
     100x100 design regions, 6000 steps, batched (several steps of all of them a launch, CUDA-
-    graph chunks, tile shape by size) against the same instances run one at a time: through the
-    3D engine (``one_at_a_time``) and as batches of one on the same TE kernel and tile shape
+    graph chunks, tile shape as the batch chooses it) against the same instances run one at a time: through
+    ``Simulation.run`` (``one_at_a_time``) and as batches of one on the same TE kernel and tile shape
     (``one_at_a_time_te_kernel``, which isolates the batching's own gain)."""
     from photonoxide_b200.batch import Batch
     steps = args.batch_steps
