@@ -1646,16 +1646,20 @@ int block_shape(const std::vector<InstanceView> &views, int sms) {
 // The tile shape of a batch whose caller fixed none; *sure: whether sizes alone tell, or the shapes had better
 // be timed. Sizes tell in f32 where the tiles of several steps are few (up to two an SM a step is its launches:
 // 16 grids of 64 x 64 5.0 us a step and 6.7 with the best of one step) or at least 65 % full (256 grids of
-// 100 x 100, 69 %: 53 and 70), and in f64 where more than four an SM are at least 85 % full (above: 10.4 M cells
-// in 35 209 and 266). Between, either may be the faster by half: f32, 256 grids of 64 x 64, 43 % full, 37 against
+// 100 x 100, 69 %: 53 and 70), and in f64 where they are at least 85 % full and more than four an SM (10.4 M
+// cells in 35 209 and 266), or fewer while as full tiles of one step are four an SM or more (0.16 M cells 16.9
+// and 11.4; as long at 1.3 M). Between, either may be the faster by half: f32, 256 grids of 64 x 64, 43 % full, 37 against
 // 28, of 136 x 136, 48 %, 115 against 130; f64, 256 of 100 x 100, 69 %, 145 against 111, 1024 of 32 x 32 272
 // against 49; f64 and small, 64 grids and fewer, which one-step shape is best changes too.
 int choose_shape(const std::vector<InstanceView> &views, int sms, bool *sure) {
   const int block = block_shape(views, sms);
   if (views[0].precision == 64) {
-    *sure = count_tiles(views, BLOCK_LARGE) > 4LL * sms && fill(views, BLOCK_LARGE) >= 0.85;
-    if (*sure) return BLOCK_LARGE;
-    return fill(views, ONE_STEP) >= 0.8 ? ONE_STEP : ONE_STEP_NARROW;
+    const bool many = count_tiles(views, BLOCK_LARGE) > 4LL * sms;
+    const double full = fill(views, ONE_STEP);
+    *sure = many ? fill(views, BLOCK_LARGE) >= 0.85
+                 : full >= 0.85 && count_tiles(views, ONE_STEP) >= 4LL * sms;
+    if (*sure) return many ? BLOCK_LARGE : ONE_STEP;
+    return full >= 0.8 ? ONE_STEP : ONE_STEP_NARROW;
   }
   *sure = count_tiles(views, BLOCK_SMALL) <= 2LL * sms || fill(views, block) >= 0.65;
   return *sure || fill(views, block) >= 0.5 ? block : ONE_STEP_NARROW;
