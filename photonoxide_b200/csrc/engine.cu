@@ -2467,6 +2467,9 @@ struct fdtd_ctx {
   fdtd_batch *solo = nullptr;
   size_t solo_held = 0;  // the bytes of its tables, in `used` too
   unsigned long long solo_refused = ~0ULL;  // the layout its tables had no room in
+  // the layout of its tables, and the steps asked for since the layout last changed (solo_worth)
+  unsigned long long solo_made = ~0ULL, solo_seen = ~0ULL;
+  long long solo_steps = 0;
   int te = 0;
   bool forced = false;  // a kernel was asked for by name
   int stride() const { return nwaves + naux + nbloch; }
@@ -2979,8 +2982,8 @@ bool solo_ok(const fdtd_ctx *c, long long steps) {
   if (c->n[2] != 1 || !c->periodic[2] || c->media || c->nbloch > 0) return false;
   // f64, where a tile has half the warps, with CPMLs: up to here the quad kernel's step is the shorter (us a step,
   // tiles and quad: 201 x 100 17 and 14, 400 x 300 15.9 and 15.1, 500 x 400 16.0 and 18.9, 1000 x 800 26 and 56;
-  // between walls 400 x 300 3.5 and 14)
-  if (c->precision == 64 && c->N < 180000 && c->low[0] + c->high[0] + c->low[1] + c->high[1] > 0) return false;
+  // between walls 400 x 300 3.5 and 14); with probes, whose runs have no graph there, 300 x 200 19.3 and 20.3
+  if (c->precision == 64 && c->N < 180000 && c->nprobes == 0 && c->low[0] + c->high[0] + c->low[1] + c->high[1] > 0) return false;
   // a caller that captures the stream: the general kernels' launches are all it can hold
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
@@ -2989,6 +2992,17 @@ bool solo_ok(const fdtd_ctx *c, long long steps) {
   for (const fdtd_injection &x : c->src_inj)
     if ((x.field == 1) != (x.component == 2) && x.point != 2) return false;
   return true;
+}
+
+// Whether the TE tiles' tables are worth making for this layout: each monitored value costs the host some 30 ns
+// of them and saves some 30 ps a step, so they wait until a thousandth as many steps have been asked for as
+// there are values. (A 300 x 200 plane's transform, a probe added before every 50 steps: 14.4 ms a time with
+// the tables made anew, 11.1 without. A 400 x 200 plane: 10 ms to make them, 12 us a step against 26.)
+bool solo_worth(fdtd_ctx *c, long long steps) {
+  if (c->solo_seen != c->layout) c->solo_steps = 0;
+  c->solo_seen = c->layout;
+  c->solo_steps += steps;
+  return (c->solo && c->solo_made == c->layout) || c->nvalues <= 1000 * c->solo_steps;
 }
 
 template <typename T>
@@ -3000,7 +3014,7 @@ int run_impl(fdtd_ctx *c, long long steps, long long first) {
   if (c->nbloch > 0)
     return fail(c, FDTD_E_STATE, "a context with Bloch couplings steps with fdtd_bloch_run");
   c->sums_fresh = true;
-  if (solo_ok(c, steps)) {
+  if (solo_ok(c, steps) && solo_worth(c, steps)) {
     bool te = false;
     double *rows = nullptr;
     if (int r = fdtd_instance_reserve(c, steps, &rows)) return r;
@@ -3011,6 +3025,7 @@ int run_impl(fdtd_ctx *c, long long steps, long long first) {
     c->solo_held = held;
     if (te) {
       c->te = 1;
+      c->solo_made = c->layout;
       return r == 0 ? 0 : fail(c, r, "a run on the TE tiles: %s", fdtd_batch_last_error(c->solo));
     }
     if (r) {  // no room for its tables: nothing has run, and the general path serves

@@ -6,6 +6,7 @@ import gc
 import numpy as np
 import pytest
 
+from photonoxide_b200.engine import Engine
 from photonoxide_b200.fdtd import Simulation
 from photonoxide_b200.types import Axis, Boundaries, Boxes, Field, Grid3d, Source, Waveform
 
@@ -66,13 +67,18 @@ def test_short_rings_and_chunks_of_half_the_length(monkeypatch):
     """Transforms whose ring the engine's 1 GB cuts to 8 rows (the tiles' chunks are of 16 steps: half of
     the plane's values stay zero in a TE run): the general kernels' bits."""
     def big():
-        s = Simulation(Grid3d.centred((2001, 1500, 1), 0.04), Boxes(2.0), Boundaries.cpml_2d(8), 0.7)
+        s = Simulation(Grid3d.centred((1001, 1500, 1), 0.04), Boxes(2.0), Boundaries.cpml_2d(8), 0.7, precision=64)
         s.add_source(Source(Field.H, Axis.Z, (200, 150, 0), Waveform.pulse(1.0, 0.6)))
-        s.add_dft((0, 0, 0), (2000, 1499, 0), [0.9])
-        s.run(51)
+        s.add_dft((0, 0, 0), (1000, 1499, 0), [0.9])
+        for steps in (40, 8992, 51):  # the tables wait for a thousandth of the 9 million values' steps
+            s.run(steps)
+            counts.append(Engine(s.engine()).launches() / steps)
         return s.h(2), s.transforms()
 
+    counts = []
     a = big()
     monkeypatch.setenv("PHOTONOXIDE_FDTD_KERNEL", "quad")
     b = big()
+    general, tiles = counts[0], counts[2]
+    assert tiles < 0.7 * general and counts[5] > 0.9 * general  # (a launch a step, and the recording's)
     assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
