@@ -2980,10 +2980,14 @@ void launch_aux(fdtd_ctx *c, int stride, long long first, const long long *base,
 bool solo_ok(const fdtd_ctx *c, long long steps) {
   if (c->solo_refused == c->layout || c->forced || c->profiling || c->capturing || steps < SOLO_STEPS || c->te < 0) return false;
   if (c->n[2] != 1 || !c->periodic[2] || c->media || c->nbloch > 0) return false;
-  // f64, where a tile has half the warps, with CPMLs: up to here the quad kernel's step is the shorter (us a step,
-  // tiles and quad: 201 x 100 17 and 14, 400 x 300 15.9 and 15.1, 500 x 400 16.0 and 18.9, 1000 x 800 26 and 56;
-  // between walls 400 x 300 3.5 and 14); with probes, whose runs have no graph there, 300 x 200 19.3 and 20.3
-  if (c->precision == 64 && c->N < 180000 && c->nprobes == 0 && c->low[0] + c->high[0] + c->low[1] + c->high[1] > 0) return false;
+  // f64, where a tile has half the warps, with a CPML along y (four values of psi a lane and row there): while the
+  // quad kernel's CTAs are one an SM or fewer its step is the shorter (us a step, tiles and quad: 201 x 100 17
+  // and 14, 301 x 201 17.0 and 14.1; but 500 x 400 16.0 and 18.9, 16 x 4000 26 and 50, 1000 x 800 26 and 56, 400
+  // x 1 periodic along y 6 and 8, 400 x 300 between walls 3.5 and 14); not with probes, whose runs have no graph
+  // there (300 x 200 19.3 and 20.3)
+  if (c->precision == 64 && c->nprobes == 0 && c->low[1] + c->high[1] > 0 &&
+      (long long)c->tiles_x * c->tiles_y <= c->sms)
+    return false;
   // a caller that captures the stream: the general kernels' launches are all it can hold
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
